@@ -608,8 +608,10 @@ extern "C" int mg_optimize_layout(const mg_layout_args* a) {
                     a->mid_w1, s);
         }
         sgd_copy_back(*a, c, s);
-        if (any_host({a->Y, a->epoch_of_next_sample, a->epoch_of_next_negative_sample, a->adam_m}))
-            MGB_CUDA(cudaStreamSynchronize(s));
+        if (any_host({a->Y, a->epoch_of_next_sample, a->epoch_of_next_negative_sample, a->adam_m})) {
+            if (a->parallel == 1) owner_finish(*g_sgd_work, s);
+            else MGB_CUDA(cudaStreamSynchronize(s));
+        }
     });
 }
 

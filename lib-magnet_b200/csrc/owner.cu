@@ -7,19 +7,23 @@
 // layout as it was at the start of the epoch; with the reverse mid pairs, u also takes, after each edge, the pulls
 // of the nodes that chose it. The result is a function of the inputs alone, whatever the thread count.
 //
-// On the device one epoch is four steps on the caller's stream:
-//  1. snapshot: the layout (and the Adam state) is copied aside; it is the "start of the epoch" every read uses;
-//  2. schedule, one thread per edge: advances eons / eonns as the reference does and records each sampled edge's
-//     negatives count; then the chain pass, one warp per chunk: consumes the chunk's stream in edge order as
-//     the edge loop would (n_neg draws, the mid-range test and walk, the reverse-pull draws), recording at each
-//     head's first sampled edge the stream state where its draws start. It reads no position: the draws depend
-//     on positions only through a negative at distance 0 exactly (src/layout.cpp:181), which draws dim extra
-//     uniforms;
-//  3. node pass, one thread per head node: from its recorded state, replays the node's edges as the reference
-//     does (other positions from the snapshot, its own in registers) and writes its row. A negative at distance 0
-//     marks the node's chunk, since the states recorded after it are then off by dim draws;
-//  4. fallback, one thread per chunk, doing work for marked chunks only: restores the rows of the chunk's heads
-//     (and their Adam state) from the snapshot and replays the whole chunk serially from the chunk's seed.
+// On the device the schedule and the draws of a batch of epochs run ahead of the positions, because they depend on
+// them only through a negative at distance 0 exactly (src/layout.cpp:181), which draws dim extra uniforms:
+//  1. schedule, one thread per edge: advances eons / eonns over the batch's epochs as the reference does and records
+//     each epoch's negatives count per sampled edge;
+//  2. chain, one thread or warp per (epoch, chunk): consumes the chunk's stream in edge order as the edge loop would (n_neg
+//     draws, the mid-range test and walk, the reverse-pull draws), recording at each head's first sampled edge the
+//     stream state where its draws start. It reads no position.
+// Then each epoch, from a read buffer into a write buffer that swap from epoch to epoch (two copies of the layout, of
+// which only rows with edges are ever written):
+//  3. node pass: replays every head's edges as the reference does from the head's recorded state (other positions
+//     from the read buffer, its own in registers) and writes its row. A negative at distance 0 marks the node's
+//     chunk, since the states recorded after it are then off by dim draws;
+//  4. fallback, one thread per chunk, doing work for marked chunks only: replays the whole chunk serially from the
+//     chunk's seed.
+// Epochs without mid-range pulls in 2-d under the power kernel and the sgd optimizer (every transform) run steps 3
+// and 4 of a whole batch in one cooperative launch with a grid barrier between epochs (owner_epochs_kernel); other
+// epochs launch the two steps one by one, Adam's with its state and the layout copied aside first.
 // This file is compiled without FMA contraction (-fmad=false): every product and sum rounds on its own, as in
 // the reference's plain x86-64 build. The power kernel with b = rep_b = 1 under the sgd optimizer uses +, *, / and
 // sqrt only and reproduces the reference bit for bit; powf, expf, tanhf and coshf may differ from the host libm
@@ -40,7 +44,7 @@ struct OwnerDev {
     const int64_t* row;                                       // first edge of each node (n + 1 entries)
     const int32_t* rev_indptr; const int32_t* rev_indices;    // reverse mid pairs or NULL
     int32_t* n_neg;                                           // per edge: this epoch's negatives, kNotSampled
-    uint64_t* node_state;                                     // stream state at each node's first edge
+    uint64_t* state;                                          // stream state of a head, at its first edge
     int* dirty;                                               // per chunk: a distance-0 negative was drawn
     const float* Yr;                                          // the layout at the start of the epoch
     const float* snap_m; const float* snap_v; const int32_t* snap_t;   // the Adam state at the start
@@ -233,6 +237,208 @@ __device__ uint64_t owner_node(const SgdDev& c, const OwnerDev& o, int64_t u, ui
     return r.s;
 }
 
+// ---------------------------------------------------------------------------------------------- pipelined node pass
+// Each head by a group of 1 to 8 lanes, with owner_node's arithmetic in its order, for the common case (2-d, power
+// kernel, no per-node b, sgd, no mid-range pulls). What depends on no position runs ahead: the group's first lane lists
+// the row's sampled edges in shared memory and makes their draws, as many edges as fit the head's kSlots positions (a
+// round: the whole row, as a rule); then all positions of the round are copied into shared memory at once (cp.async),
+// and the edges computed from there one after another, an edge's negatives by the group's lanes side by side, their
+// terms added in the negatives' order by every lane. A head so waits for one L2 read per round; owner_node waits for
+// one per negative, 37 us per epoch of a 48-row transform. Per epoch of the same transform other forms took 17 us (one
+// lane per head: the negatives' divisions one after another) and 14 us (8 lanes, each repeating the whole stream's
+// 64-bit steps to keep its own draw).
+constexpr int kEpochThreads = 128;
+constexpr int kRowList = 32;    // edges of a row listed at a time
+constexpr int kSlots = 48;      // positions of a round
+
+__device__ __forceinline__ float2 ld2(const float* Y, int64_t u) {
+    return __ldcg(reinterpret_cast<const float2*>(Y) + u);   // rows other SMs wrote in the previous epoch
+}
+
+// what a step reads besides positions, kept in registers over a launch's epochs
+struct OwnerCoef {
+    float a, b, rep_a, rep_b, two_b, att;   // att = -1.5 * exaggeration * 2 a b, in the reference's order of products
+    bool b_one, rep_b_one, norm_clip;
+    __device__ __forceinline__ explicit OwnerCoef(const SgdDev& c)
+        : a(c.a), b(c.b), rep_a(c.rep_a), rep_b(c.rep_b), two_b(c.two_b),
+          att(-kOwnerAttraction * c.exaggeration * 2.0f * c.a * c.b), b_one(c.b_is_one), rep_b_one(c.rep_b_is_one),
+          norm_clip(c.clip_mode == 1) {}
+};
+
+// one negative at yk; at distance 0 the reference draws jitter, which marks the chunk for the replay
+__device__ __forceinline__ void add_negative(const OwnerCoef& c, float2 yu, float2 yk, float2& gu, bool& jitter) {
+    const float dx = yu.x - yk.x, dy = yu.y - yk.y;
+    const float dd = dx * dx + dy * dy;
+    if (dd > 0.0f) {
+        const float pw = c.rep_b_one ? dd : powf(dd, c.rep_b);
+        const float coeff = c.two_b / ((0.001f + dd) * (c.rep_a * pw + 1.0f));
+        gu.x += coeff * dx; gu.y += coeff * dy;
+    } else {
+        jitter = true;
+    }
+}
+
+__device__ __forceinline__ void xorshift(uint64_t& s) { s ^= s >> 12; s ^= s << 25; s ^= s >> 27; }   // Rng::next() without its output
+__device__ __forceinline__ int32_t below_state(uint64_t s, int64_t n) {
+    return (int32_t)((((s * 0x2545F4914F6CDD1DULL) >> 32) * (uint64_t)(uint32_t)n) >> 32);
+}
+
+__device__ __forceinline__ void copy8(float2* dst, const float2* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copies_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+struct EpochShared {
+    int2 edge[kRowList][kEpochThreads];       // (negatives, tail) of the listed edges
+    int32_t index[kSlots][kEpochThreads];     // the round's rows: per edge its tail, then its negatives (-1: the head itself)
+    float2 pos[kSlots][kEpochThreads];        // their positions
+};
+
+// the walk over a head's sampled edges, in the head's own column of the shared arrays (held by the group's first lane)
+struct HeadWalk {
+    int col;
+    int64_t row1, w0;
+    int have, taken;        // edges listed, edges taken by rounds so far
+    int first, used;        // the round: its first edge in the list, its slots
+    bool wide;              // the round is one edge of more negatives than the slots hold: drawn as it is computed
+    uint64_t stream;
+
+    __device__ __forceinline__ void fill(const int32_t* __restrict__ rec, const int32_t* __restrict__ tails, EpochShared& sh) {
+        const int cnt = (int)(row1 - w0 < kRowList ? row1 - w0 : kRowList);
+        have = 0; taken = 0;
+        for (int t0 = 0; t0 < cnt; t0 += 8) {
+            int nn[8], tt[8];
+#pragma unroll
+            for (int t = 0; t < 8; ++t) {
+                nn[t] = t0 + t < cnt ? rec[w0 + t0 + t] : kNotSampled;
+                tt[t] = t0 + t < cnt ? tails[w0 + t0 + t] : 0;
+            }
+#pragma unroll
+            for (int t = 0; t < 8; ++t)
+                if (nn[t] != kNotSampled) sh.edge[have++][col] = make_int2(nn[t], tt[t]);
+        }
+    }
+    // the next round's edges and draws; false when the row has ended
+    __device__ __forceinline__ bool round(const int32_t* __restrict__ rec, const int32_t* __restrict__ tails, int64_t u,
+                                          int64_t n_nodes, EpochShared& sh) {
+        while (taken == have && w0 + kRowList < row1) { w0 += kRowList; fill(rec, tails, sh); }
+        first = taken; used = 0; wide = false;
+        while (taken < have) {
+            const int2 e = sh.edge[taken][col];
+            const int nn = e.x > 0 ? e.x : 0;
+            if (used + 1 + nn > kSlots) {
+                if (used > 0) break;
+                wide = true;
+                sh.index[0][col] = e.y;
+                used = 1;
+                ++taken;
+                break;
+            }
+            sh.index[used++][col] = e.y;
+            for (int t = 0; t < nn; ++t) {
+                xorshift(stream);
+                const int32_t k = below_state(stream, n_nodes);
+                sh.index[used++][col] = k != (int32_t)u ? k : -1;
+            }
+            ++taken;
+        }
+        return taken > first;
+    }
+};
+
+// the heads of a warp's groups of G lanes (has: the group has one, u), walks started and first rounds made by the
+// groups' first lanes (more: the round has edges); the groups step together. Returns whether this lane met a
+// distance-0 negative.
+__device__ __forceinline__ bool owner_heads(const OwnerCoef& c, const float* __restrict__ Yr, float* __restrict__ Yw,
+                                            const int32_t* __restrict__ rec, const int32_t* __restrict__ tails,
+                                            int64_t n, int64_t n_fixed, int64_t u, bool has, HeadWalk& walk, bool more,
+                                            float alpha, EpochShared& sh, int G) {
+    constexpr unsigned kFull = 0xffffffffu;
+    const int lane = threadIdx.x & 31, gl = lane & (G - 1), lead = lane - gl, col = threadIdx.x / G;
+    bool jitter = false;
+    const bool move_u = has && u >= n_fixed;
+    float2 yu = make_float2(0.0f, 0.0f);
+    if (has) yu = ld2(Yr, u);
+    const float cap = 4.0f * alpha;
+    for (;;) {
+        const bool go = __shfl_sync(kFull, (int)(has && more), lead) != 0;
+        if (!__any_sync(kFull, go)) break;
+        const int first = __shfl_sync(kFull, walk.first, lead);
+        const int edges = go ? __shfl_sync(kFull, walk.taken, lead) - first : (__shfl_sync(kFull, walk.taken, lead), 0);
+        const int used = __shfl_sync(kFull, walk.used, lead);
+        const bool wide = __shfl_sync(kFull, (int)walk.wide, lead) != 0;
+        if (go)
+            for (int q = gl; q < used; q += G) {
+                const int32_t k = sh.index[q][col];
+                if (k >= 0) copy8(&sh.pos[q][col], reinterpret_cast<const float2*>(Yr) + k);
+            }
+        copies_done();
+        __syncwarp();
+        int at = 0;
+        for (int e = 0; __any_sync(kFull, e < edges); ++e) {
+            const bool act = e < edges;
+            float2 gu = make_float2(0.0f, 0.0f);
+            int nn = 0;
+            if (act) {
+                nn = max(sh.edge[first + e][col].x, 0);
+                const float2 yv = sh.pos[at++][col];
+                if (!wide)
+                    for (int t = gl; t < nn; t += G) {
+                        if (sh.index[at + t][col] < 0) continue;
+                        float2 term = make_float2(0.0f, 0.0f);
+                        bool zero = false;
+                        add_negative(c, yu, sh.pos[at + t][col], term, zero);
+                        sh.pos[at + t][col] = term;
+                        if (zero) { jitter = true; sh.index[at + t][col] = -1; }
+                    }
+                const float dx = yu.x - yv.x, dy = yu.y - yv.y;
+                const float d2 = dx * dx + dy * dy;
+                if (d2 > 0.0f) {
+                    const float pw_v = c.b_one ? d2 : powf(d2, c.b);
+                    const float coeff = c.att * pw_v / (d2 * (c.a * pw_v + 1.0f));
+                    gu.x += coeff * dx; gu.y += coeff * dy;
+                }
+            }
+            __syncwarp();
+            if (act && !wide) {
+#pragma unroll 4
+                for (int t = 0; t < nn; ++t, ++at) {
+                    const float2 term = sh.pos[at][col];
+                    if (sh.index[at][col] >= 0) { gu.x += term.x; gu.y += term.y; }
+                }
+            }
+            if (__any_sync(kFull, act && wide)) {
+                if (act && wide && gl == 0)
+                    for (int t = 0; t < nn; ++t) {
+                        xorshift(walk.stream);
+                        const int32_t k = below_state(walk.stream, n);
+                        if (k != (int32_t)u) add_negative(c, yu, ld2(Yr, k), gu, jitter);
+                    }
+                gu.x = __shfl_sync(kFull, gu.x, wide ? lead : lane);
+                gu.y = __shfl_sync(kFull, gu.y, wide ? lead : lane);
+            }
+            if (act && move_u) {
+                // apply_step (src/layout.cpp:90-116), as owner_step
+                float sx = alpha * gu.x, sy = alpha * gu.y;
+                if (c.norm_clip) {
+                    float n2 = 0.0f;
+                    n2 += sx * sx; n2 += sy * sy;
+                    if (n2 > cap * cap) { const float f = cap / sqrtf(n2); sx *= f; sy *= f; }
+                } else {
+                    sx = sx > cap ? cap : (sx < -cap ? -cap : sx);
+                    sy = sy > cap ? cap : (sy < -cap ? -cap : sy);
+                }
+                yu.x += sx; yu.y += sy;
+            }
+        }
+        __syncwarp();   // the round's columns are read no more
+        if (has && more && gl == 0) more = walk.round(rec, tails, u, n, sh);
+        __syncwarp();
+    }
+    if (move_u && gl == 0) reinterpret_cast<float2*>(Yw)[u] = yu;
+    return jitter;
+}
+
 // ---------------------------------------------------------------------------------------------- set-up kernels
 // first edge of every node (lower bound of u in the sorted heads), u in [0, n]
 __global__ void owner_rows_kernel(const int32_t* __restrict__ head, int64_t E, int64_t n, int64_t* __restrict__ row) {
@@ -263,41 +469,144 @@ __global__ void owner_sorted_kernel(const int32_t* __restrict__ head, int64_t E,
         if (head[i - 1] > head[i]) { atomicExch(unsorted, 1); return; }
 }
 
-// ---------------------------------------------------------------------------------------------- epoch kernels
-// the epoch's schedule, one thread per edge (coalesced): eons / eonns advanced as src/layout.cpp:135,160-163,184
-// advance them, and each edge's negatives count recorded (kNotSampled when eons[i] > epoch)
-__global__ void __launch_bounds__(256) owner_schedule_kernel(SgdDev c, OwnerDev o, int epoch) {
-    const float fepoch = (float)epoch;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < c.n_edges;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const float eo = c.eons[i];
-        if (eo > fepoch) { o.n_neg[i] = kNotSampled; continue; }
-        const float ep = c.eps[i];
-        c.eons[i] = eo + ep;
-        const float epn = ep / c.negative_sample_rate;
-        const float en = c.eonns[i];
-        const int n_neg = (int)((fepoch - en) / epn);
-        c.eonns[i] = en + (float)n_neg * epn;
-        o.n_neg[i] = n_neg;
+// the heads (edges that start a row), in no order; for layouts whose fixed rows mostly have no edges
+__global__ void owner_heads_kernel(const int32_t* __restrict__ head, int64_t E, int32_t* __restrict__ list,
+                                   int* __restrict__ count) {
+    const int lane = threadIdx.x & 31;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t base = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < E; base += stride) {
+        const int64_t i = base + lane;
+        const bool first = i < E && (i == 0 || head[i] != head[i - 1]);
+        const unsigned m = __ballot_sync(0xffffffffu, first);
+        int at = 0;
+        if (lane == 0 && m) at = atomicAdd(count, __popc(m));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (first) list[at + __popc(m & ((1u << lane) - 1u))] = head[i];
     }
 }
 
-// One warp per chunk: the chunk's stream consumed in edge order from the recorded negatives counts. The lanes
-// read 32 edges' counts and heads at a time (coalesced) and take the sampled ones in order from a ballot; every
-// lane holds the same stream state and makes the same draws, so control flow stays uniform across the warp.
-// A head's state is recorded at its first sampled edge (edges that are not sampled draw nothing, and a head
-// without sampled edges draws nothing in the node pass), so heads without edges, such as the fixed training rows
-// of a transform, cost nothing. No position is read and nothing is stored but the per-node states.
-constexpr int kChainWarps = 4;   // chunks per block
+// ---------------------------------------------------------------------------------------------- epoch kernels
+// run_epochs' linear schedule inside a call (src/layout.cpp:284-289), as sgd_sched evaluates it on the host
+struct OwnerSched {
+    int e0, n_span;
+    float alpha0, alpha1, mid_w0, mid_w1;
+    bool use_mid;
+    __device__ __forceinline__ float frac(int epoch) const { return (float)(epoch - e0) / (float)n_span; }
+    __device__ __forceinline__ float alpha(int epoch) const { return alpha0 + (alpha1 - alpha0) * frac(epoch); }
+    __device__ __forceinline__ float mid_w(int epoch) const {
+        return use_mid ? mid_w0 + (mid_w1 - mid_w0) * frac(epoch) : 0.0f;
+    }
+};
 
-__global__ void __launch_bounds__(32 * kChainWarps) owner_chain_kernel(SgdDev c, OwnerDev o, int epoch,
-                                                                        float mid_w) {
-    const int k = blockIdx.x * kChainWarps + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (k >= o.n_chunks) return;
+// the schedule of epochs [b0, b0 + B), one thread per edge (coalesced): eons / eonns advanced as
+// src/layout.cpp:135,160-163,184 advance them, and each epoch's negatives count recorded (kNotSampled when
+// eons[i] > epoch)
+__global__ void __launch_bounds__(256) owner_schedule_kernel(SgdDev c, int32_t* __restrict__ rec, int b0, int B) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < c.n_edges;
+         i += (int64_t)gridDim.x * blockDim.x) {
+        float eo = c.eons[i], en = c.eonns[i];
+        const float ep = c.eps[i];
+        const float epn = ep / c.negative_sample_rate;
+        for (int k = 0; k < B; ++k) {
+            const float fepoch = (float)(b0 + k);
+            int n_neg = kNotSampled;
+            if (!(eo > fepoch)) {
+                eo = eo + ep;
+                n_neg = (int)((fepoch - en) / epn);
+                en = en + (float)n_neg * epn;
+            }
+            rec[(int64_t)k * c.n_edges + i] = n_neg;
+        }
+        c.eons[i] = eo;
+        c.eonns[i] = en;
+    }
+}
+
+// The chain pass. A head's state is recorded at its first sampled edge (edges that are not sampled draw nothing, and
+// a head without sampled edges draws nothing in the node pass), so heads without edges, such as the fixed training
+// rows of a transform, cost nothing. No position is read and nothing is stored but the heads' states.
+// Two forms, by the edges per chunk:
+//  * owner_chain_kernel, one thread per (chunk, epoch of the batch), consecutive threads on consecutive epochs of the
+//    same chunk: they walk the same rows, so their draws between two heads come together. For the short chunks of a
+//    transform (256 edges); a warp each, launched per epoch, took 25-28 us per epoch;
+//  * owner_chain_warp_kernel, one warp per (chunk, epoch): the lanes read 32 edges' counts and heads at a time and
+//    take the sampled ones in order from a ballot; every lane holds the same stream state. For the reference's chunks
+//    of 4096 edges and more, of which a batch has too few for a thread each (0.46 ms per epoch of the 1M-point
+//    graph, several ms with a thread each).
+constexpr int kChainThreads = 64;
+constexpr int kChainWarps = 4;                    // chunks per block of the warp form
+constexpr int64_t kChainThreadMaxEdges = 1024;    // mean edges per chunk up to which the thread form runs
+
+__global__ void __launch_bounds__(kChainThreads) owner_chain_kernel(SgdDev c, OwnerDev o, OwnerSched sc, int b0, int B) {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (int64_t)B * o.n_chunks) return;
+    const int k = (int)(t / B), be = (int)(t - (int64_t)k * B);
+    const int epoch = b0 + be;
+    const float mid_w = sc.mid_w(epoch);
     Rng r(stream_seed(c.seed, epoch, (uint64_t)k));
     const float inv_n_mid = c.n_mid > 0 ? 1.0f / (float)c.n_mid : 0.0f;
-    const int32_t* __restrict__ rec = o.n_neg;
+    const int32_t* __restrict__ rec = o.n_neg + (int64_t)be * c.n_edges;
+    uint64_t* __restrict__ state = o.state + (int64_t)be * c.n_edges;
+    const int64_t e0 = o.eown[k], e1 = o.eown[k + 1];
+    int64_t row_start = e0;
+    int32_t u = -1, done = -1;   // the head walked, the head whose state is recorded
+    int pend = 0;                // negatives' draws not made yet (made when the state is needed)
+    float p0 = 0.0f;
+    constexpr int kAhead = 8;
+    int32_t nn[kAhead], hh[kAhead];
+    auto fetch = [&](int64_t base) {
+#pragma unroll
+        for (int q = 0; q < kAhead; ++q) {
+            nn[q] = base + q < e1 ? __ldg(rec + base + q) : kNotSampled;
+            hh[q] = base + q < e1 ? __ldg(c.head + base + q) : u;
+        }
+    };
+    auto draw_pending = [&]() {
+        for (; pend > 0; --pend) xorshift(r.s);
+    };
+    if (e0 < e1) fetch(e0);
+    for (int64_t base = e0; base < e1; base += kAhead) {
+        int32_t cn[kAhead], ch[kAhead];
+#pragma unroll
+        for (int q = 0; q < kAhead; ++q) { cn[q] = nn[q]; ch[q] = hh[q]; }
+        if (base + kAhead < e1) fetch(base + kAhead);
+#pragma unroll
+        for (int q = 0; q < kAhead; ++q) {
+            if (base + q >= e1) break;
+            if (ch[q] != u) { u = ch[q]; row_start = base + q; draw_pending(); }
+            if (cn[q] == kNotSampled) continue;
+            if (u != done) {
+                done = u;
+                state[row_start] = r.s;
+                // the reverse-pull rounds of each of u's edges: the same p for every edge of u
+                p0 = 0.0f;
+                if (u >= c.n_fixed && mid_w > 0.0f && o.rev_indptr) {
+                    const int32_t rs = o.rev_indptr[u], re = o.rev_indptr[u + 1];
+                    if (re > rs) p0 = c.mid_rate * (float)(re - rs) * inv_n_mid;
+                }
+            }
+            pend += cn[q] > 0 ? cn[q] : 0;
+            if (mid_w > 0.0f) {
+                draw_pending();
+                if (r.uniform() < c.mid_rate) (void)mid_partner(c, r, u, c.tail[base + q]);
+                for (float p = p0; p > 0.0f; p -= 1.0f)
+                    if (r.uniform() < p) (void)r.next();
+            }
+        }
+    }
+}
+
+__global__ void __launch_bounds__(32 * kChainWarps) owner_chain_warp_kernel(SgdDev c, OwnerDev o, OwnerSched sc, int b0, int B) {
+    const int64_t t = (int64_t)blockIdx.x * kChainWarps + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    if (t >= (int64_t)B * o.n_chunks) return;
+    const int be = (int)(t / o.n_chunks), k = (int)(t - (int64_t)be * o.n_chunks);
+    const int epoch = b0 + be;
+    const float mid_w = sc.mid_w(epoch);
+    Rng r(stream_seed(c.seed, epoch, (uint64_t)k));
+    const float inv_n_mid = c.n_mid > 0 ? 1.0f / (float)c.n_mid : 0.0f;
+    const int32_t* __restrict__ rec = o.n_neg + (int64_t)be * c.n_edges;
+    uint64_t* __restrict__ state = o.state + (int64_t)be * c.n_edges;
     const int64_t e0 = o.eown[k], e1 = o.eown[k + 1];
     int64_t u = -1;
     float p0 = 0.0f;
@@ -313,7 +622,7 @@ __global__ void __launch_bounds__(32 * kChainWarps) owner_chain_kernel(SgdDev c,
             const int32_t h = __shfl_sync(0xffffffffu, my_head, b);
             if (h != u) {
                 u = h;
-                if (lane == 0) o.node_state[u] = r.s;
+                if (lane == 0) state[o.row[u]] = r.s;
                 // the reverse-pull rounds of each of u's edges: the same p for every edge of u
                 p0 = 0.0f;
                 if (u >= c.n_fixed && mid_w > 0.0f && o.rev_indptr) {
@@ -321,7 +630,7 @@ __global__ void __launch_bounds__(32 * kChainWarps) owner_chain_kernel(SgdDev c,
                     if (re > rs) p0 = c.mid_rate * (float)(re - rs) * inv_n_mid;
                 }
             }
-            for (int p = 0; p < n_neg; ++p) r.next();
+            for (int p = 0; p < n_neg; ++p) xorshift(r.s);
             if (mid_w > 0.0f && r.uniform() < c.mid_rate) (void)mid_partner(c, r, u, c.tail[base + b]);
             for (float p = p0; p > 0.0f; p -= 1.0f)
                 if (r.uniform() < p) (void)r.next();
@@ -329,30 +638,30 @@ __global__ void __launch_bounds__(32 * kChainWarps) owner_chain_kernel(SgdDev c,
     }
 }
 
-template <int D>
-__global__ void __launch_bounds__(128) owner_node_kernel(SgdDev c, OwnerDev o, int epoch, float alpha, float mid_w) {
-    const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (u >= c.n || o.row[u] == o.row[u + 1]) return;
-    bool jitter = false;
-    owner_node<D>(c, o, u, o.node_state[u], alpha, mid_w, jitter);
-    if (jitter) {
-        // the chunk holding u: the last k with own[k] <= u (empty chunks share their bound with the next one)
-        int lo = 0, hi = o.n_chunks;
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (o.own[mid] <= u) lo = mid; else hi = mid;
-        }
-        atomicExch(&o.dirty[lo], 1);
+// the chunk holding u: the last k with own[k] <= u (empty chunks share their bound with the next one)
+__device__ __forceinline__ int chunk_of(const OwnerDev& o, int64_t u) {
+    int lo = 0, hi = o.n_chunks;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (o.own[mid] <= u) lo = mid; else hi = mid;
     }
+    return lo;
 }
 
 template <int D>
-__global__ void __launch_bounds__(32) owner_fallback_kernel(SgdDev c, OwnerDev o, int epoch, float alpha,
-                                                            float mid_w) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= o.n_chunks || !o.dirty[k]) return;
-    o.dirty[k] = 0;
-    // the heads of the chunk's edges (a marked chunk has at least one); rows without edges never move
+__global__ void __launch_bounds__(128) owner_node_kernel(SgdDev c, OwnerDev o, float alpha, float mid_w) {
+    const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (u >= c.n || o.row[u] == o.row[u + 1]) return;
+    bool jitter = false;
+    owner_node<D>(c, o, u, o.state[o.row[u]], alpha, mid_w, jitter);
+    if (jitter) atomicExch(&o.dirty[chunk_of(o, u)], 1);
+}
+
+// the marked chunk k replayed serially from its seed; rows without edges never move
+template <int D>
+__device__ __noinline__ void owner_replay(const SgdDev& c, const OwnerDev& o, int k, int epoch, float alpha,
+                                          float mid_w) {
+    // the heads of the chunk's edges (a marked chunk has at least one)
     const int64_t u0 = c.head[o.eown[k]], u1 = (int64_t)c.head[o.eown[k + 1] - 1] + 1;
     const int dim = c.dim;
     for (int64_t j = u0 * dim; j < u1 * dim; ++j) c.Y[j] = o.Yr[j];
@@ -366,12 +675,164 @@ __global__ void __launch_bounds__(32) owner_fallback_kernel(SgdDev c, OwnerDev o
 }
 
 template <int D>
+__global__ void __launch_bounds__(32) owner_fallback_kernel(SgdDev c, OwnerDev o, int epoch, float alpha,
+                                                            float mid_w) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= o.n_chunks || !o.dirty[k]) return;
+    o.dirty[k] = 0;
+    owner_replay<D>(c, o, k, epoch, alpha, mid_w);
+}
+
+template <int D>
 void owner_epoch_launch(const SgdDev& c, const OwnerDev& o, int epoch, float alpha, float mid_w, cudaStream_t s) {
-    owner_node_kernel<D><<<ceil_div(c.n, 128), 128, 0, s>>>(c, o, epoch, alpha, mid_w);
+    owner_node_kernel<D><<<ceil_div(c.n, 128), 128, 0, s>>>(c, o, alpha, mid_w);
     MGB_LAUNCH_CHECK();
     owner_fallback_kernel<D><<<ceil_div(o.n_chunks, 32), 32, 0, s>>>(c, o, epoch, alpha, mid_w);
     MGB_LAUNCH_CHECK();
 }
+
+// Grid barrier of a cooperative launch, in two halves: every block arrives on a counter that only grows, then waits for
+// all. The wait gives up after about a second (never reached while the launch's blocks run), sets *err and lets the
+// kernel end.
+struct GridBarrier {
+    unsigned* count;
+    int* err;
+    unsigned passed = 0;
+    __device__ __forceinline__ void arrive() {
+        ++passed;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            atomicAdd(count, 1u);
+        }
+    }
+    __device__ __forceinline__ bool wait() {
+        __shared__ int ok;
+        if (threadIdx.x == 0) {
+            const unsigned want = passed * gridDim.x;
+            int tries = 0;
+            int good = 1;
+            while (*reinterpret_cast<volatile unsigned*>(count) < want)
+                if (++tries > 4000000 || *reinterpret_cast<volatile int*>(err)) { atomicExch(err, 1); good = 0; break; }
+            __threadfence();
+            ok = good;
+        }
+        __syncthreads();
+        return ok != 0;
+    }
+};
+
+// epoch `epoch`'s marked chunks, replayed by the grid's threads (its records at rec / state, layout Yr -> Yw)
+__device__ __noinline__ void owner_replay_marked(const SgdDev& call, const OwnerDev& own, int epoch, float alpha,
+                                                 const float* Yr, float* Yw, int32_t* rec, uint64_t* state) {
+    SgdDev c = call;
+    OwnerDev o = own;
+    c.Y = Yw;
+    o.Yr = Yr; o.n_neg = rec; o.state = state;
+    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < o.n_chunks; q += (int64_t)gridDim.x * blockDim.x)
+        if (__ldcg(&o.dirty[q])) {
+            o.dirty[q] = 0;
+            owner_replay<2>(c, o, (int)q, epoch, alpha, 0.0f);
+        }
+}
+
+// Epochs [b0, b0 + B) of the pipelined node pass in one cooperative launch: epoch k reads buffer k & 1 and writes the
+// other; a grid barrier separates the epochs, and a second one follows the fallback of an epoch that marked a chunk.
+// Bound by the latency of one epoch (one L2 read, the steps of the longest row, the barrier).
+// 14 us per epoch of a 48-row transform and 18 of a 4096-row one, where the five operations per epoch before it took
+// 68 and 76 (200k fixed rows, 14 edges per row, 100 epochs).
+// Few heads are spread thin, by groups of G lanes (G a power of two up to 8): as long as every scheduler has a warp.
+__global__ void __launch_bounds__(kEpochThreads) owner_epochs_kernel(const __grid_constant__ SgdDev c,
+                                                           const __grid_constant__ OwnerDev o, OwnerSched sc, int b0, int B,
+                                                           int G, float* buf0, float* buf1,
+                                                           const int32_t* __restrict__ heads,
+                                                           const int* __restrict__ n_heads, int* __restrict__ any_dirty,
+                                                           unsigned* bar, int* err) {
+    extern __shared__ __align__(16) unsigned char epoch_smem[];
+    EpochShared& sh = *reinterpret_cast<EpochShared*>(epoch_smem);
+    const int gl = threadIdx.x & (G - 1);
+    const int64_t groups = (int64_t)gridDim.x * (blockDim.x / G);
+    const int64_t work = heads ? *n_heads : c.n;
+    const int64_t g0 = (int64_t)blockIdx.x * (blockDim.x / G) + threadIdx.x / G;
+    const int64_t gw = (int64_t)blockIdx.x * (blockDim.x / G) + (threadIdx.x & ~31) / G;   // the warp's first group
+    const OwnerCoef coef(c);
+    const int64_t n = c.n, n_fixed = c.n_fixed, E = c.n_edges;
+    const int32_t* const tail = c.tail;
+    const int64_t* const row = o.row;
+    GridBarrier barrier{bar, err};
+    // one head per group (every transform): its row bounds stay in registers, and the first round of an epoch is made
+    // between the two halves of the barrier that ends the epoch before
+    const bool single = work <= groups;
+    int64_t u = -1, row0 = 0, row1 = 0;
+    HeadWalk walk{};
+    walk.col = threadIdx.x / G;
+    bool more = false, has = false;
+    auto head_at = [&](int64_t h) {
+        u = heads ? (int64_t)heads[h] : h;
+        row0 = row[u];
+        row1 = row[u + 1];
+        has = row0 < row1;
+    };
+    auto begin = [&](int k) {
+        const int32_t* rec = o.n_neg + (int64_t)k * E;
+        walk.w0 = row0; walk.row1 = row1;
+        walk.stream = o.state[(int64_t)k * E + row0];   // used when an edge of the row is sampled
+        walk.fill(rec, tail, sh);
+        more = walk.round(rec, tail, u, n, sh);
+    };
+    if (single && g0 < work) {
+        head_at(g0);
+        if (has && gl == 0) begin(0);
+    }
+    __syncwarp();
+    for (int k = 0; k < B; ++k) {
+        const int epoch = b0 + k;
+        const float alpha = sc.alpha(epoch);
+        const float* const Yr = (k & 1) ? buf1 : buf0;
+        float* const Yw = (k & 1) ? buf0 : buf1;
+        for (int64_t hw = gw; hw < work; hw += groups) {   // uniform in the warp
+            if (!single) {
+                const int64_t h = hw + (threadIdx.x & 31) / G;
+                has = false;
+                if (h < work) head_at(h);
+                if (has && gl == 0) begin(k);
+                __syncwarp();
+            }
+            if (owner_heads(coef, Yr, Yw, o.n_neg + (int64_t)k * E, tail, n, n_fixed, u, has, walk, more, alpha, sh, G)) {
+                atomicExch(&o.dirty[chunk_of(o, u)], 1);
+                atomicExch(&any_dirty[k], 1);
+            }
+        }
+        barrier.arrive();
+        if (single && has && gl == 0 && k + 1 < B) begin(k + 1);
+        if (!barrier.wait()) return;
+        if (__ldcg(&any_dirty[k])) {
+            owner_replay_marked(c, o, epoch, alpha, Yr, Yw, o.n_neg + (int64_t)k * E, o.state + (int64_t)k * E);
+            barrier.arrive();
+            if (!barrier.wait()) return;
+        }
+    }
+}
+
+// resident blocks of owner_epochs_kernel, asked once per thread and device
+int owner_resident_blocks() {
+    static thread_local int dev_known = -1, blocks = 0;
+    int dev = 0;
+    MGB_CUDA(cudaGetDevice(&dev));
+    if (dev != dev_known) {
+        int per_sm = 0;
+        MGB_CUDA(cudaFuncSetAttribute((const void*)owner_epochs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)sizeof(EpochShared)));
+        MGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, owner_epochs_kernel, kEpochThreads,
+                                                               sizeof(EpochShared)));
+        blocks = std::max(1, per_sm) * kNumSMs;
+        dev_known = dev;
+    }
+    return blocks;
+}
+
+// bytes of records (negatives counts and head states, 12 per edge and epoch) that a batch of epochs may hold
+constexpr int64_t kOwnerAheadBytes = 96LL << 20;
 
 }  // namespace
 
@@ -380,16 +841,39 @@ int owner_chunk_count(int64_t n_edges, int chunk_edges) {
     return (int)std::min<int64_t>(chunk_edges > 0 ? INT32_MAX / 2 : 4096, std::max<int64_t>(1, n_edges / per));
 }
 
+// the call's flags: [0] unsorted heads, [1] a grid barrier of an earlier call gave up
+static int* owner_flags(SgdWork& w, cudaStream_t s) {
+    const bool fresh = w.flag.p == nullptr;
+    int* flag = static_cast<int*>(w.flag.ensure(2 * sizeof(int)));
+    if (fresh || !w.flags_ready) MGB_CUDA(cudaMemsetAsync(flag, 0, 2 * sizeof(int), s));
+    w.flags_ready = true;
+    return flag;
+}
+
+static void owner_check_timeout(int gave_up, SgdWork& w, cudaStream_t s) {
+    if (!gave_up) return;
+    MGB_CUDA(cudaMemsetAsync(w.flag.as<int>() + 1, 0, sizeof(int), s));
+    throw Error(MG_ERR_TIMEOUT, "owner mode: a grid barrier gave up; the layout of that call is not valid");
+}
+
 bool owner_heads_sorted(const int32_t* head_dev, int64_t n_edges, SgdWork& w, cudaStream_t s) {
     if (n_edges < 2) return true;
-    int* flag = static_cast<int*>(w.flag.ensure(sizeof(int)));
+    int* flag = owner_flags(w, s);
     MGB_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), s));
     owner_sorted_kernel<<<std::min(ceil_div(n_edges, 256), 4 * kNumSMs), 256, 0, s>>>(head_dev, n_edges, flag);
     MGB_LAUNCH_CHECK();
-    int h = 0;
-    MGB_CUDA(cudaMemcpyAsync(&h, flag, sizeof(int), cudaMemcpyDeviceToHost, s));
+    int h[2] = {0, 0};
+    MGB_CUDA(cudaMemcpyAsync(h, flag, sizeof(h), cudaMemcpyDeviceToHost, s));
     MGB_CUDA(cudaStreamSynchronize(s));
-    return h == 0;
+    owner_check_timeout(h[1], w, s);
+    return h[0] == 0;
+}
+
+void owner_finish(SgdWork& w, cudaStream_t s) {
+    int gave_up = 0;
+    MGB_CUDA(cudaMemcpyAsync(&gave_up, owner_flags(w, s) + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
+    MGB_CUDA(cudaStreamSynchronize(s));
+    owner_check_timeout(gave_up, w, s);
 }
 
 void owner_run(SgdDev& c, SgdWork& w, const int32_t* rev_indptr, const int32_t* rev_indices, int chunk_edges,
@@ -397,21 +881,28 @@ void owner_run(SgdDev& c, SgdWork& w, const int32_t* rev_indptr, const int32_t* 
     const int64_t n = c.n, E = c.n_edges;
     const int dim = c.dim;
     const int nc = owner_chunk_count(E, chunk_edges);
+    const size_t y_bytes = sizeof(float) * (size_t)(n * dim);
     OwnerDev o{};
     int64_t* row = static_cast<int64_t*>(w.o_row.ensure(sizeof(int64_t) * (n + 1)));
     int64_t* own = static_cast<int64_t*>(w.o_own.ensure(sizeof(int64_t) * (nc + 1) * 2));
     int64_t* eown = own + (nc + 1);
     o.row = row; o.own = own; o.eown = eown; o.n_chunks = nc;
     o.rev_indptr = rev_indptr; o.rev_indices = rev_indices;
-    o.n_neg = static_cast<int32_t*>(w.o_neg.ensure(sizeof(int32_t) * std::max<int64_t>(E, 1)));
-    o.node_state = static_cast<uint64_t*>(w.o_state.ensure(sizeof(uint64_t) * std::max<int64_t>(n, 1)));
+    // epochs whose schedule and draws are made together: as many as the records' bound allows
+    const int64_t per_epoch = 12 * std::max<int64_t>(E, 1);
+    const int ahead = (int)std::max<int64_t>(1, std::min<int64_t>(e1 - e0, kOwnerAheadBytes / per_epoch));
+    // (sized a quarter above the call's edges: the next request of about the same rows keeps the buffers)
+    const size_t room = (size_t)((E + E / 4 + 1) * ahead);
+    int32_t* rec = static_cast<int32_t*>(w.o_neg.ensure(sizeof(int32_t) * room));
+    uint64_t* state = static_cast<uint64_t*>(w.o_state.ensure(sizeof(uint64_t) * room));
     o.dirty = static_cast<int*>(w.o_dirty.ensure(sizeof(int) * nc));
-    float* snap = static_cast<float*>(w.o_snap.ensure(sizeof(float) * std::max<int64_t>(n * dim, 1)));
-    o.Yr = snap;
+    float* snap = static_cast<float*>(w.o_snap.ensure(std::max<size_t>(y_bytes, sizeof(float))));
+    float* const Y = c.Y;
+    const bool adam = c.optimizer == 1;
     float* snap_m = nullptr; float* snap_v = nullptr; int32_t* snap_t = nullptr;
-    if (c.optimizer == 1) {
-        snap_m = static_cast<float*>(w.o_snap_m.ensure(sizeof(float) * std::max<int64_t>(n * dim, 1)));
-        snap_v = static_cast<float*>(w.o_snap_v.ensure(sizeof(float) * std::max<int64_t>(n * dim, 1)));
+    if (adam) {
+        snap_m = static_cast<float*>(w.o_snap_m.ensure(std::max<size_t>(y_bytes, sizeof(float))));
+        snap_v = static_cast<float*>(w.o_snap_v.ensure(std::max<size_t>(y_bytes, sizeof(float))));
         snap_t = static_cast<int32_t*>(w.o_snap_t.ensure(sizeof(int32_t) * std::max<int64_t>(n, 1)));
     }
     o.snap_m = snap_m; o.snap_v = snap_v; o.snap_t = snap_t;
@@ -420,21 +911,86 @@ void owner_run(SgdDev& c, SgdWork& w, const int32_t* rev_indptr, const int32_t* 
     MGB_LAUNCH_CHECK();
     owner_chunks_kernel<<<ceil_div(nc + 1, 256), 256, 0, s>>>(c.head, E, n, nc, row, own, eown);
     MGB_LAUNCH_CHECK();
-    for (int epoch = e0; epoch < e1; ++epoch) {
-        float alpha, mid_w;
-        sgd_sched(c, epoch, e0, e1, alpha0, alpha1, mid_w0, mid_w1, alpha, mid_w);
-        MGB_CUDA(cudaMemcpyAsync(snap, c.Y, sizeof(float) * n * dim, cudaMemcpyDeviceToDevice, s));
-        if (c.optimizer == 1) {
-            MGB_CUDA(cudaMemcpyAsync(snap_m, c.adam_m, sizeof(float) * n * dim, cudaMemcpyDeviceToDevice, s));
-            MGB_CUDA(cudaMemcpyAsync(snap_v, c.adam_v, sizeof(float) * n * dim, cudaMemcpyDeviceToDevice, s));
-            MGB_CUDA(cudaMemcpyAsync(snap_t, c.adam_t, sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, s));
+    OwnerSched sc{e0, std::max(1, e1 - e0), alpha0, alpha1, mid_w0, mid_w1, c.use_mid};
+    // the pipelined node pass: 8-byte aligned 2-d rows, the power kernel without per-node b, plain steps, and heads
+    // that the device holds at once (more take turns in a block's few warps: 0.68 against 0.55 ms per epoch at 300k
+    // rows of 24 edges, where 20k rows take 0.08 against 0.28)
+    const int64_t rows = c.n_fixed > 0 ? std::min<int64_t>(E, n - c.n_fixed) : n;
+    const bool pipelined = rows <= (int64_t)owner_resident_blocks() * kEpochThreads && dim == 2 && c.kernel == 0 && !c.node_b && !adam &&
+                        (reinterpret_cast<uintptr_t>(Y) % sizeof(float2)) == 0;
+    int32_t* heads = nullptr;
+    int* sync_words = nullptr;   // [0] barrier, [1] head count, [2 + k] epoch k of the batch marked a chunk
+    if (pipelined) {
+        sync_words = static_cast<int*>(w.o_sync.ensure(sizeof(int) * (size_t)(2 + ahead)));
+        MGB_CUDA(cudaMemsetAsync(sync_words, 0, sizeof(int) * 2, s));
+        if (c.n_fixed > 0) {
+            heads = static_cast<int32_t*>(w.o_heads.ensure(sizeof(int32_t) * (size_t)E));
+            owner_heads_kernel<<<std::min(ceil_div(E, 256), 4 * kNumSMs), 256, 0, s>>>(c.head, E, heads, sync_words + 1);
+            MGB_LAUNCH_CHECK();
         }
-        owner_schedule_kernel<<<std::min(ceil_div(E, 256), 8 * kNumSMs), 256, 0, s>>>(c, o, epoch);
-        MGB_LAUNCH_CHECK();
-        owner_chain_kernel<<<ceil_div(nc, kChainWarps), 32 * kChainWarps, 0, s>>>(c, o, epoch, mid_w);
-        MGB_LAUNCH_CHECK();
-        MGB_DIM_DISPATCH(dim, owner_epoch_launch, c, o, epoch, alpha, mid_w, s);
     }
+    // the two buffers of the layout: cur is read next, the other written (Adam's epochs always read the copy)
+    float* cur = Y;
+    float* other = snap;
+    if (!adam) MGB_CUDA(cudaMemcpyAsync(snap, Y, y_bytes, cudaMemcpyDeviceToDevice, s));
+    for (int b0 = e0; b0 < e1; b0 += ahead) {
+        const int B = std::min(ahead, e1 - b0);
+        owner_schedule_kernel<<<std::min(ceil_div(E, 256), 8 * kNumSMs), 256, 0, s>>>(c, rec, b0, B);
+        MGB_LAUNCH_CHECK();
+        o.n_neg = rec; o.state = state;
+        if (E <= kChainThreadMaxEdges * nc)
+            owner_chain_kernel<<<ceil_div((int64_t)B * nc, kChainThreads), kChainThreads, 0, s>>>(c, o, sc, b0, B);
+        else
+            owner_chain_warp_kernel<<<ceil_div((int64_t)B * nc, kChainWarps), 32 * kChainWarps, 0, s>>>(c, o, sc, b0, B);
+        MGB_LAUNCH_CHECK();
+        for (int k = 0; k < B;) {
+            float alpha, mid_w;
+            sgd_sched(c, b0 + k, e0, e1, alpha0, alpha1, mid_w0, mid_w1, alpha, mid_w);
+            int run = 0;   // epochs from k on without mid-range pulls
+            while (pipelined && k + run < B) {
+                float a, mw;
+                sgd_sched(c, b0 + k + run, e0, e1, alpha0, alpha1, mid_w0, mid_w1, a, mw);
+                if (mw > 0.0f) break;
+                ++run;
+            }
+            o.n_neg = rec + (int64_t)k * E;
+            o.state = state + (int64_t)k * E;
+            SgdDev cc = c;
+            if (run > 0) {
+                MGB_CUDA(cudaMemsetAsync(sync_words, 0, sizeof(int), s));
+                MGB_CUDA(cudaMemsetAsync(sync_words + 2, 0, sizeof(int) * (size_t)run, s));
+                // lanes per head: 8 while the warps are at most one per scheduler
+                int G = 8;
+                while (G > 1 && rows * G > 4LL * kNumSMs * 32) G /= 2;
+                int blocks = (int)std::min<int64_t>(owner_resident_blocks(), std::max(1, ceil_div(rows * G, kEpochThreads)));
+                int b = b0 + k;
+                const int* n_heads = sync_words + 1;
+                int* any_dirty = sync_words + 2;
+                unsigned* bar = reinterpret_cast<unsigned*>(sync_words);
+                int* err = owner_flags(w, s) + 1;
+                void* args[] = {&cc, &o, &sc, &b, &run, &G, &cur, &other, &heads, &n_heads, &any_dirty, &bar, &err};
+                MGB_CUDA(cudaLaunchCooperativeKernel((const void*)owner_epochs_kernel, dim3(blocks), dim3(kEpochThreads), args, sizeof(EpochShared), s));
+                MGB_LAUNCH_CHECK();
+                if (run & 1) std::swap(cur, other);
+                k += run;
+                continue;
+            }
+            if (adam) {
+                MGB_CUDA(cudaMemcpyAsync(snap, Y, y_bytes, cudaMemcpyDeviceToDevice, s));
+                MGB_CUDA(cudaMemcpyAsync(snap_m, c.adam_m, y_bytes, cudaMemcpyDeviceToDevice, s));
+                MGB_CUDA(cudaMemcpyAsync(snap_v, c.adam_v, y_bytes, cudaMemcpyDeviceToDevice, s));
+                MGB_CUDA(cudaMemcpyAsync(snap_t, c.adam_t, sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, s));
+                o.Yr = snap;
+            } else {
+                o.Yr = cur;
+                cc.Y = other;
+                std::swap(cur, other);
+            }
+            MGB_DIM_DISPATCH(dim, owner_epoch_launch, cc, o, b0 + k, alpha, mid_w, s);
+            ++k;
+        }
+    }
+    if (cur != Y) MGB_CUDA(cudaMemcpyAsync(Y, cur, y_bytes, cudaMemcpyDeviceToDevice, s));
 }
 
 }  // namespace mgb

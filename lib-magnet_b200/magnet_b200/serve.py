@@ -227,14 +227,16 @@ class FittedLayout:
     def request_bytes(self, m):
         """device bytes a transform of m rows holds at its peak: a block of query distances (and its padded copy
         when the tiles do not divide n), the first-stage top-k candidates, the neighbour arrays, the layout copy
-        and the SGD's per-edge and per-node scratch"""
+        and the SGD's per-edge and per-node scratch, with owner mode's records of the epochs made ahead (12 bytes per
+        edge and epoch, at most 96 MB or one epoch's, and a quarter more)"""
+        records = 15 * m * self.k * max(1, min(self.epochs, (96 << 20) // max(1, 12 * m * self.k)))
         if self.search:
-            return 12 * m * self.k + 4 * m * self.d + 64 * m * self.k + 48 * (self.n + m)
+            return 12 * m * self.k + 4 * m * self.d + 64 * m * self.k + 48 * (self.n + m) + records
         mb = min(m, self.block)
         padded = self.n_tiles * self.tile
         dist_block = 4 * mb * self.n + (4 * mb * padded if padded != self.n else 0)
         candidates = 12 * mb * self.n_tiles * self.k
-        return dist_block + candidates + 64 * m * self.k + 48 * (self.n + m)
+        return dist_block + candidates + 64 * m * self.k + 48 * (self.n + m) + records
 
     def bind_stream(self):
         """give this thread a CUDA stream of its own: torch's current stream for the thread, and the C ABI's"""
