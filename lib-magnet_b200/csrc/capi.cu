@@ -702,20 +702,19 @@ extern "C" int mg_chebyshev_eigenvectors(const int32_t* indptr, const int32_t* i
         require(n <= INT32_MAX, "n must fit 32-bit indices");
         if (p > kSpecMaxCols) throw Error(MG_ERR_NOT_SUPPORTED, "the device solver takes at most 8 columns");
         validate_csr_host(indptr, indices, nnz, n, -1, "chebyshev_eigenvectors");
-        // the component labels on the host: their count sizes the per-component sums
-        std::vector<int32_t> comp_h;
-        const int32_t* ch = component;
-        if (is_device_ptr(component)) {
-            comp_h.resize((size_t)n);
-            MGB_CUDA(cudaMemcpy(comp_h.data(), component, sizeof(int32_t) * (size_t)n, cudaMemcpyDeviceToHost));
-            ch = comp_h.data();
-        }
-        int32_t n_comp = 0;
-        for (int64_t i = 0; i < n; ++i) {
-            require(ch[i] >= 0, "component labels must be >= 0");
-            n_comp = std::max(n_comp, ch[i] + 1);
-        }
+        // the number of components sizes the per-component sums
         cudaStream_t s = current_stream();
+        int32_t range[2] = {0, -1};   // smallest and largest label
+        if (is_device_ptr(component)) {
+            label_range_dev(component, n, range, spec_work(), s);
+        } else {
+            for (int64_t i = 0; i < n; ++i) {
+                range[0] = std::min(range[0], component[i]);
+                range[1] = std::max(range[1], component[i]);
+            }
+        }
+        require(range[0] >= 0, "component labels must be >= 0");
+        const int32_t n_comp = range[1] + 1;
         const int32_t* ip = in_dev(indptr, n + 1, 0, s);
         const int32_t* ix = in_dev(indices, nnz, 1, s);
         const float* pd = in_dev(data, nnz, 2, s);

@@ -9,8 +9,8 @@ namespace mgb {
 
 constexpr int kSpecMaxCols = 8;   // columns of the block (n_wanted + extra) the device solver takes
 
-// device scratch of the solver: the block and its filter iterates (n x p FP64 each), per-component sums and
-// per-block partial sums
+// device scratch of the solver: the block and its filter iterate, each as it is and scaled by D^-1/2 (n x p FP64
+// each), per-component sums (three sets) and per-block partial sums
 struct SpecWork {
     DevBuf X, Z, Y, Ynew, proj, tnorm, part;
 };
@@ -21,6 +21,9 @@ struct SpecWork {
 void chebyshev_eigenvectors_dev(const int32_t* indptr, const int32_t* indices, const float* data, int64_t n,
                                 const float* sd, const int32_t* comp, int n_comp, float* X, int p, int n_wanted,
                                 int degree, int max_iter, double tol, SpecWork& w, cudaStream_t s);
+
+// the smallest and largest of n component labels (device array); synchronises s
+void label_range_dev(const int32_t* comp, int64_t n, int32_t range[2], SpecWork& w, cudaStream_t s);
 
 // the small symmetric eigenproblem of the Rayleigh-Ritz step (host): A (p x p, row major) -> eigenvalues in
 // descending order and the eigenvectors as the columns of V (row major)
