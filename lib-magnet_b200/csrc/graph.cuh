@@ -7,10 +7,10 @@ namespace mgb {
 
 // device scratch of the graph passes
 struct GraphWork {
-    DevBuf sigma, rho, part, acol, aval, alen, tcnt, tptr, tcur, trow, tval, ucnt, uptr, scan, flag;
+    DevBuf sigma, rho, part, acol, aval, alen, tcnt, tptr, tcur, trow, ucnt, uptr, scan, flag;
     DevBuf mid_state, mid_tab;   // mid-near partners: per-row stream states, jump tables and chunk tables
     DevBuf sched;                // the transform schedule's kept-edge count
-    DevBuf s_part, s_flag, s_off, s_tmp;   // the fit schedule's block partials, keep flags, offsets, scan tiles
+    DevBuf s_part, s_flag, s_off, s_tmp;   // the fit schedule's state and partials, row counts and offsets, scan tiles
 };
 
 // memberships (n_rows, k) of sorted neighbour distances; `target` = log2(n_neighbors) * bandwidth, computed by the
