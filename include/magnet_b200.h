@@ -122,16 +122,16 @@ void mg_tsne_params_default(mg_tsne_params* p);
 int mg_optimize_tsne(const int32_t* indptr, const int32_t* indices, const float* P, int64_t n, int64_t nnz,
                      float* Y, const mg_tsne_params* p);
 /* The same pass with per-stage timing: plain launches bracketed by CUDA events on the calling thread's stream.
- * stage_ms[9] receives the summed milliseconds of: 0 bbox + grid choice, 1 twiddles, 2 kernel spectra,
- * 3 spread, 4 forward row FFTs, 5 column FFT convolution, 6 inverse row FFTs, 7 gather + attraction + step,
- * 8 all; grid[4] receives the last iteration's (n_boxes, N, M, Mh). */
+ * stage_ms[9] receives the summed milliseconds of: 0 the first grid choice, 1 nothing (the twiddles are made with the
+ * grid), 2 kernel spectra, 3 spread, 4 forward row FFTs, 5 column FFT convolution, 6 inverse row FFTs, 7 gather +
+ * attraction + step + the next grid choice, 8 all; grid[4] receives the last iteration's (n_boxes, N, M, Mh). */
 int mg_optimize_tsne_profiled(const int32_t* indptr, const int32_t* indices, const float* P, int64_t n, int64_t nnz,
                               float* Y, const mg_tsne_params* p, double* stage_ms, int* grid);
 /* ================================================================ batched t-SNE layouts
  * Many independent optimize_tsne passes (magnet/tsne.py:132-214; the reference runs them as a loop of
  * optimize_tsne calls) of uneven size, run together: each layout keeps its own device state, and one CUDA graph
- * holds one iteration of every layout as independent branches (layout i on branch i mod `branches`), replayed
- * once per iteration. Every layout uses the same parameters p (n_iter, early_iter, schedule, n_interp, box width);
+ * holds one iteration of every layout, replayed once per iteration: its launches each cover a set of layouts, and
+ * `branches` (at least 1; more than two make no difference) sets run side by side. Every layout uses the same parameters p (n_iter, early_iter, schedule, n_interp, box width);
  * its grid is allocated for max_boxes[i] boxes per side (NULL: 64 + 2 ceil(sqrt(n_i)) rounded up to a multiple of
  * 4, capped by p->max_boxes), and a layout that outgrows it is clamped to that many boxes (wider boxes). The
  * arrays of layout i are indptr[i] (n[i] + 1), indices[i] / P[i] (nnz[i]), host or device; P is normalised to

@@ -161,15 +161,107 @@ template <int R> struct Split {
                            : (R % 5 == 0 && R != 5) ? 5 : (R % 4 == 0 && R != 4) ? 4 : (R % 3 == 0 && R != 3) ? 3 : 2;
 };
 
-// forward DFT_R in registers: base radices directly, composites R = A B by one Cooley-Tukey split
-// (n = B n1 + n2, k = k1 + A k2)
-template <int R>
-__device__ __forceinline__ void dft_fwd(float2* v) {
-    if constexpr (R == 2) fft::dft2(v);
-    else if constexpr (R == 3) fft::dft3(v);
-    else if constexpr (R == 4) fft::dft4(v);
-    else if constexpr (R == 5) fft::dft5(v);
-    else if constexpr (R == 8) fft::dft8(v);
+// Packed single-precision pairs: one instruction adds, multiplies or fuses both halves of a complex value (each half
+// rounded as the scalar operation rounds it). The butterflies are mostly complex additions, which so take half the
+// issue slots. The column pass, bound by issue and by its stages' latency, at M = 4320: 154 to 133 million warp
+// instructions, 272 to 246 us (with the buffers addressed as shared memory instead of through generic pointers).
+__device__ __forceinline__ unsigned long long pk(float2 a) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
+    return r;
+}
+__device__ __forceinline__ float2 upk(unsigned long long a) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+    return r;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pk(a)), "l"(pk(b)));
+    return upk(r);
+}
+__device__ __forceinline__ float2 mul2(float2 a, float b) {
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pk(a)), "l"(pk(make_float2(b, b))));
+    return upk(r);
+}
+__device__ __forceinline__ float2 fma2(float2 a, float b, float2 c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(pk(a)), "l"(pk(make_float2(b, b))), "l"(pk(c)));
+    return upk(r);
+}
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return fma2(b, -1.f, a); }   // exact product
+
+// a -+ i b: forward (INV = false) a - i b, inverse a + i b, and the other sign
+template <bool INV>
+__device__ __forceinline__ float2 add_rot(float2 a, float2 b) {
+    return INV ? make_float2(a.x - b.y, a.y + b.x) : make_float2(a.x + b.y, a.y - b.x);
+}
+template <bool INV>
+__device__ __forceinline__ float2 sub_rot(float2 a, float2 b) { return add_rot<!INV>(a, b); }
+// a -+ i s b, one rounding
+template <bool INV>
+__device__ __forceinline__ float2 fma_rot(float2 b, float s, float2 a) {
+    return INV ? make_float2(fmaf(-s, b.y, a.x), fmaf(s, b.x, a.y)) : make_float2(fmaf(s, b.y, a.x), fmaf(-s, b.x, a.y));
+}
+
+template <bool INV>
+__device__ __forceinline__ void base2(float2* v) {
+    const float2 a = v[0], b = v[1];
+    v[0] = add2(a, b); v[1] = sub2(a, b);
+}
+template <bool INV>
+__device__ __forceinline__ void base3(float2* v) {
+    const float s3 = 0.86602540378443864676f;
+    const float2 t1 = add2(v[1], v[2]), t2 = sub2(v[1], v[2]);
+    const float2 m = fma2(t1, -0.5f, v[0]);
+    v[0] = add2(v[0], t1);
+    v[1] = fma_rot<INV>(t2, s3, m);
+    v[2] = fma_rot<INV>(t2, -s3, m);
+}
+template <bool INV>
+__device__ __forceinline__ void base4(float2* v) {
+    const float2 a = add2(v[0], v[2]), b = sub2(v[0], v[2]);
+    const float2 c = add2(v[1], v[3]), d = sub2(v[1], v[3]);
+    v[0] = add2(a, c); v[2] = sub2(a, c);
+    v[1] = add_rot<INV>(b, d); v[3] = sub_rot<INV>(b, d);
+}
+template <bool INV>
+__device__ __forceinline__ void base5(float2* v) {
+    const float c1 = 0.30901699437494742410f, c2 = -0.80901699437494742410f;
+    const float s1 = 0.95105651629515357212f, s2 = 0.58778525229247312917f;
+    const float2 t1 = add2(v[1], v[4]), t2 = add2(v[2], v[3]);
+    const float2 t3 = sub2(v[1], v[4]), t4 = sub2(v[2], v[3]);
+    const float2 x0 = v[0];
+    const float2 a1 = fma2(t2, c2, fma2(t1, c1, x0)), a2 = fma2(t2, c1, fma2(t1, c2, x0));
+    const float2 b1 = fma2(t4, s2, mul2(t3, s1)), b2 = fma2(t4, -s1, mul2(t3, s2));
+    v[0] = add2(x0, add2(t1, t2));
+    v[1] = add_rot<INV>(a1, b1); v[4] = sub_rot<INV>(a1, b1);
+    v[2] = add_rot<INV>(a2, b2); v[3] = sub_rot<INV>(a2, b2);
+}
+template <bool INV>
+__device__ __forceinline__ void base8(float2* v) {
+    const float h = 0.70710678118654752440f;
+    float2 e[4] = {v[0], v[2], v[4], v[6]};
+    float2 o[4] = {v[1], v[3], v[5], v[7]};
+    base4<INV>(e); base4<INV>(o);
+    // o_1 and o_3 times w8 and w8^3, w8 = exp(-+ i pi / 4), the factor h fused into the sums; o_2 times -+ i in the sums
+    const float2 r1 = add_rot<INV>(o[1], o[1]), r3 = sub_rot<INV>(o[3], o[3]);
+    v[0] = add2(e[0], o[0]); v[4] = sub2(e[0], o[0]);
+    v[1] = fma2(r1, h, e[1]); v[5] = fma2(r1, -h, e[1]);
+    v[2] = add_rot<INV>(e[2], o[2]); v[6] = sub_rot<INV>(e[2], o[2]);
+    v[3] = fma2(r3, -h, e[3]); v[7] = fma2(r3, h, e[3]);
+}
+
+// DFT_R in registers, forward or (unnormalised) inverse: base radices directly, composites R = A B by one Cooley-Tukey
+// split (n = B n1 + n2, k = k1 + A k2)
+template <int R, bool INV>
+__device__ __forceinline__ void dft(float2* v) {
+    if constexpr (R == 2) base2<INV>(v);
+    else if constexpr (R == 3) base3<INV>(v);
+    else if constexpr (R == 4) base4<INV>(v);
+    else if constexpr (R == 5) base5<INV>(v);
+    else if constexpr (R == 8) base8<INV>(v);
     else {
         constexpr int A = Split<R>::A, B = R / A;
         float2 y[R];
@@ -178,7 +270,7 @@ __device__ __forceinline__ void dft_fwd(float2* v) {
             float2 t[A];
 #pragma unroll
             for (int n1 = 0; n1 < A; ++n1) t[n1] = v[B * n1 + n2];
-            dft_fwd<A>(t);
+            dft<A, INV>(t);
 #pragma unroll
             for (int k1 = 0; k1 < A; ++k1) y[n2 * A + k1] = t[k1];
         }
@@ -188,7 +280,7 @@ __device__ __forceinline__ void dft_fwd(float2* v) {
             static_for<A>([&](auto k1c) {
                 constexpr int k1 = decltype(k1c)::value;
                 if constexpr (n2 * k1 != 0) {
-                    constexpr float c = (float)cx_cos(n2 * k1, R), s = -(float)cx_sin(n2 * k1, R);
+                    constexpr float c = (float)cx_cos(n2 * k1, R), s = (INV ? 1.f : -1.f) * (float)cx_sin(n2 * k1, R);
                     const float2 a = y[n2 * A + k1];
                     y[n2 * A + k1] = make_float2(a.x * c - a.y * s, a.x * s + a.y * c);
                 }
@@ -199,22 +291,14 @@ __device__ __forceinline__ void dft_fwd(float2* v) {
             float2 t[B];
 #pragma unroll
             for (int n2 = 0; n2 < B; ++n2) t[n2] = y[n2 * A + k1];
-            dft_fwd<B>(t);
+            dft<B, INV>(t);
 #pragma unroll
             for (int k2 = 0; k2 < B; ++k2) v[k1 + A * k2] = t[k2];
         }
     }
 }
-
-// inverse (unnormalised) DFT_R: conj(DFT(conj(v)))
-template <int R>
-__device__ __forceinline__ void dft_inv(float2* v) {
-#pragma unroll
-    for (int r = 0; r < R; ++r) v[r].y = -v[r].y;
-    dft_fwd<R>(v);
-#pragma unroll
-    for (int r = 0; r < R; ++r) v[r].y = -v[r].y;
-}
+template <int R> __device__ __forceinline__ void dft_fwd(float2* v) { dft<R, false>(v); }
+template <int R> __device__ __forceinline__ void dft_inv(float2* v) { dft<R, true>(v); }
 
 #define MGB_FFT3_RADIX_DISPATCH(R, F, ...)          \
     switch (R) {                                    \
@@ -233,24 +317,37 @@ __device__ __forceinline__ void dft_inv(float2* v) {
         default: F<20>(__VA_ARGS__); break;         \
     }
 
-// v[q] *= w^q for q >= 1 (CONJ: conj(w)^q), w = tw[step]: powers by successive products from one table read,
-// re-read from the table every 8 powers so that the rounding of the recurrence stays within a few ulps
+// w^q = tw[step q] (conjugated)
+template <bool CONJ>
+__device__ __forceinline__ float2 root(const float2* __restrict__ tw, int at) {
+    float2 w = __ldg(&tw[at]);
+    if (CONJ) w.y = -w.y;
+    return w;
+}
+
+// v[q] *= w^q for q >= 1 (CONJ: conj(w)^q), w = tw[step]. Every fourth power is read from the table, the others are one
+// product away from it (w^(4a-1) = w^(4a) conj(w), w^(4a+1) = w^(4a) w, w^(4a+2) = w^(4a) w^2), with no chain to wait
+// for. The roots' errors are the larger part of a transform's: with the recurrence w^q = w^(q-1) w, restarted every 8
+// powers, F came out 8 to 18 % further from 64 bits (M = 120 to 1875), for 3 % less time.
 template <int R, bool CONJ>
 __device__ __forceinline__ void twiddle(float2* v, const float2* __restrict__ tw, int step) {
-    float2 w = __ldg(&tw[step]);
-    if (CONJ) w.y = -w.y;
-    float2 wq = w;
+    const float2 w1 = root<CONJ>(tw, step);
+    v[1] = fft::cmul(v[1], w1);
+    if constexpr (R > 2) {
+        const float2 w2 = fft::cmul(w1, w1);
+        v[2] = fft::cmul(v[2], w2);
+        if constexpr (R == 4) v[3] = fft::cmul(v[3], fft::cmul(w2, w1));
+        if constexpr (R > 4) {
+            const float2 back = make_float2(w1.x, -w1.y);
 #pragma unroll
-    for (int q = 1; q < R; ++q) {
-        if (q > 1) {
-            if (q % 8 == 0) {
-                wq = __ldg(&tw[step * q]);
-                if (CONJ) wq.y = -wq.y;
-            } else {
-                wq = fft::cmul(wq, w);
+            for (int a = 4; a <= R; a += 4) {
+                const float2 wa = root<CONJ>(tw, step * (a == R ? a - 1 : a));
+                v[a - 1] = fft::cmul(v[a - 1], a == R ? wa : fft::cmul(wa, back));
+                if (a < R) v[a] = fft::cmul(v[a], wa);
+                if (a + 1 < R) v[a + 1] = fft::cmul(v[a + 1], fft::cmul(wa, w1));
+                if (a + 2 < R) v[a + 2] = fft::cmul(v[a + 2], fft::cmul(wa, w2));
             }
         }
-        v[q] = fft::cmul(v[q], wq);
     }
 }
 
@@ -258,6 +355,13 @@ __device__ __forceinline__ void twiddle(float2* v, const float2* __restrict__ tw
 // Each stage function is compiled once per radix (not inlined), processes one or two buffers in one loop over
 // nbuf * M / R butterflies, and is shared by every call site: a plan executes a handful of small functions, which
 // keeps the instruction working set of a block inside the instruction cache.
+
+// The buffers are the block's dynamic shared memory, named by offsets: a pointer handed to a function that is not inlined
+// is a generic one, 64 bits to compute and slower to read.
+__device__ __forceinline__ float2* buffers() {
+    extern __shared__ float2 fft3_buffers[];
+    return fft3_buffers;
+}
 
 // Butterfly geometry of stage st for butterfly b: its offset j in the block and its padded start.
 __device__ __forceinline__ void bfly_at(int padR, unsigned mpad, const Stage& st, int b, int& j, int& base) {
@@ -269,7 +373,7 @@ __device__ __forceinline__ void bfly_at(int padR, unsigned mpad, const Stage& st
 
 // forward stage 1 from global memory: element n < n_live of transform t read as load(t, n), zero past it
 template <int R, class Load>
-__device__ __noinline__ void dif_first(const Plan& p, float2* __restrict__ A, float2* __restrict__ B, int nbuf,
+__device__ __noinline__ void dif_first(const Plan& p, int offA, int offB, int nbuf,
                                        Load load, int n_live, const float2* __restrict__ tw) {
     const Stage st = p.st[0];
     const int padR = p.padR;
@@ -277,7 +381,7 @@ __device__ __noinline__ void dif_first(const Plan& p, float2* __restrict__ A, fl
     for (int i = threadIdx.x; i < st.nb * nbuf; i += blockDim.x) {
         const int t = i >= st.nb ? 1 : 0;
         const int b = i - t * st.nb;
-        float2* buf = t ? B : A;
+        float2* buf = buffers() + (t ? offB : offA);
         float2 v[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) {
@@ -294,14 +398,14 @@ __device__ __noinline__ void dif_first(const Plan& p, float2* __restrict__ A, fl
 
 // forward stage s (1 <= s < S - 1) over shared memory, in place
 template <int R>
-__device__ __noinline__ void dif_mid(const Plan& p, int s, float2* __restrict__ A, float2* __restrict__ B, int nbuf,
+__device__ __noinline__ void dif_mid(const Plan& p, int s, int offA, int offB, int nbuf,
                                      const float2* __restrict__ tw) {
     const Stage st = p.st[s];
     const int padR = p.padR;
     const unsigned mpad = p.mpad;
     for (int i = threadIdx.x; i < st.nb * nbuf; i += blockDim.x) {
         const int t = i >= st.nb ? 1 : 0;
-        float2* buf = t ? B : A;
+        float2* buf = buffers() + (t ? offB : offA);
         int j, base;
         bfly_at(padR, mpad, st, i - t * st.nb, j, base);
         float2 v[R];
@@ -316,14 +420,14 @@ __device__ __noinline__ void dif_mid(const Plan& p, int s, float2* __restrict__ 
 
 // inverse stage s (1 <= s < S - 1) over shared memory, in place
 template <int R>
-__device__ __noinline__ void dit_mid(const Plan& p, int s, float2* __restrict__ A, float2* __restrict__ B, int nbuf,
+__device__ __noinline__ void dit_mid(const Plan& p, int s, int offA, int offB, int nbuf,
                                      const float2* __restrict__ tw) {
     const Stage st = p.st[s];
     const int padR = p.padR;
     const unsigned mpad = p.mpad;
     for (int i = threadIdx.x; i < st.nb * nbuf; i += blockDim.x) {
         const int t = i >= st.nb ? 1 : 0;
-        float2* buf = t ? B : A;
+        float2* buf = buffers() + (t ? offB : offA);
         int j, base;
         bfly_at(padR, mpad, st, i - t * st.nb, j, base);
         float2 v[R];
@@ -338,7 +442,7 @@ __device__ __noinline__ void dit_mid(const Plan& p, int s, float2* __restrict__ 
 
 // inverse stage 1 to global memory: element n < n_live of transform t written as store(t, n, value)
 template <int R, class Store>
-__device__ __noinline__ void dit_last(const Plan& p, const float2* __restrict__ A, const float2* __restrict__ B,
+__device__ __noinline__ void dit_last(const Plan& p, int offA, int offB,
                                       int nbuf, Store store, int n_live, const float2* __restrict__ tw) {
     const Stage st = p.st[0];
     const int padR = p.padR;
@@ -346,7 +450,7 @@ __device__ __noinline__ void dit_last(const Plan& p, const float2* __restrict__ 
     for (int i = threadIdx.x; i < st.nb * nbuf; i += blockDim.x) {
         const int t = i >= st.nb ? 1 : 0;
         const int b = i - t * st.nb;
-        const float2* buf = t ? B : A;
+        const float2* buf = buffers() + (t ? offB : offA);
         const int base = padR ? b + udiv(b, mpad) : b;
         float2 v[R];
 #pragma unroll

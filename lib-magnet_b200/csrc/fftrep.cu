@@ -347,12 +347,17 @@ __global__ void twiddle_kernel(const GridDesc* __restrict__ gd, float2* __restri
 }
 
 // Row spectra of the two kernels (rows a in [0, M/2], the kernels being even in a): z_b = K1(a,b) + i K2(a,b)
-// on the wrapped offsets of magnet/tsne.py:57-67, one complex FFT, separated; stored transposed.
-__global__ void __launch_bounds__(kFftThreads) spec_rows_kernel(const GridDesc* __restrict__ gd,
-                                                                 float2* __restrict__ Rt, int Pa, int Mhmax,
-                                                                 const float2* __restrict__ tw, int ni, double dof) {
+// on the wrapped offsets of magnet/tsne.py:57-67, one complex FFT, separated; stored transposed. Layout blockIdx.y; a
+// layout whose grid did not change is left alone. At dof 1 K2 is 1 / base^2 by one division (a general power took 60 %
+// of the two kernels' time).
+__global__ void __launch_bounds__(kFftThreads) spec_rows_kernel(const __grid_constant__ LoopArgs args) {
+    const LoopDesc L = args.many ? args.many[blockIdx.y] : args.one;
+    const GridDesc* gd = L.g;
     if (!gd->spec_dirty) return;
-    const double width_d = gd->spec_width;
+    const double width_d = gd->spec_width, dof = L.dof;
+    const int ni = L.sch.ni, Pa = L.Mmax / 2 + 1, Mhmax = L.Mhmax;
+    const float2* tw = L.tw;
+    float2* Rt = L.Rt;
     extern __shared__ float2 sm[];
     const int M = gd->M, Mh = gd->Mh;
     fft::Plan plan;
@@ -367,7 +372,7 @@ __global__ void __launch_bounds__(kFftThreads) spec_rows_kernel(const GridDesc* 
             const double ob = (double)(b <= M / 2 ? b : b - M) * delta;
             const double base = 1.0 + (oa * oa + ob * ob) / dof;
             float k1, k2;
-            if (dof == 1.0) { k1 = (float)(1.0 / base); k2 = (float)pow(base, -2.0); }
+            if (dof == 1.0) { k1 = (float)(1.0 / base); k2 = (float)(1.0 / (base * base)); }
             else { k1 = (float)pow(base, -dof); k2 = (float)pow(base, -dof - 1.0); }
             A[b] = make_float2(k1, k2);
         }
@@ -383,11 +388,12 @@ __global__ void __launch_bounds__(kFftThreads) spec_rows_kernel(const GridDesc* 
 }
 
 // Column transforms of the row spectra (mirrored to the full torus), real part kept: Kt[kern][k2][k1]
-__global__ void __launch_bounds__(kFftThreads) spec_cols_kernel(const GridDesc* __restrict__ gd,
-                                                                 const float2* __restrict__ Rt, int Pa, int Mhmax,
-                                                                 float* __restrict__ Kt, int Mmax,
-                                                                 const float2* __restrict__ tw) {
+__global__ void __launch_bounds__(kFftThreads) spec_cols_kernel(const __grid_constant__ LoopArgs args) {
+    const LoopDesc L = args.many ? args.many[blockIdx.y] : args.one;
+    const GridDesc* gd = L.g;
     if (!gd->spec_dirty) return;
+    const int Pa = L.Mmax / 2 + 1, Mhmax = L.Mhmax;
+    const float2* Rt = L.Rt;
     extern __shared__ float2 sm[];
     const int M = gd->M, Mh = gd->Mh;
     fft::Plan plan;
@@ -399,8 +405,8 @@ __global__ void __launch_bounds__(kFftThreads) spec_cols_kernel(const GridDesc* 
         const float2* src = Rt + ((size_t)kern * Mhmax + k) * Pa;
         for (int a = threadIdx.x; a < M; a += blockDim.x) A[a] = src[a <= M / 2 ? a : M - a];
         __syncthreads();
-        const float2* R = fft::forward(A, B, plan, tw, threadIdx.x, blockDim.x, BlockSync());
-        float* dst = Kt + ((size_t)kern * Mhmax + k) * Mmax;
+        const float2* R = fft::forward(A, B, plan, L.tw, threadIdx.x, blockDim.x, BlockSync());
+        float* dst = L.Kt + ((size_t)kern * Mhmax + k) * L.Mmax;
         for (int a = threadIdx.x; a < M; a += blockDim.x) dst[a] = R[a].x;
         __syncthreads();
     }
@@ -496,14 +502,24 @@ void ensure_fft_attrs() {
     done_dev = dev;
 }
 
-void rep_convolve(GridDesc* g, RepBuffers& b, int64_t n, cudaStream_t s, cudaEvent_t* ev) {
+LoopDesc rep_desc(RepBuffers& b, GridDesc* g, int64_t n) {
+    LoopDesc d{};
+    d.g = g;
+    d.W = b.W.as<float4>(); d.WhT = b.WhT.as<float2>(); d.PhT = b.PhT.as<float2>(); d.phi = b.phi.as<float>();
+    d.Kt = b.Kt.as<float>(); d.Rt = b.Rt.as<float2>(); d.tw = b.tw.as<float2>();
+    d.plans = b.plans3.as<fft3::Plan>(); d.zpart = b.zpart.as<double>(); d.fft_len = b.fft_len_table.as<int>();
+    d.Nmax = b.Nmax; d.Npmax = b.Npmax; d.Mhmax = b.Mhmax; d.Mmax = b.Mmax;
+    d.n = n;
+    return d;
+}
+
+void rep_convolve(GridDesc* g, RepBuffers& b, int64_t n, cudaStream_t s) {
     if (b.use3) {
-        rep_row_fwd3(g, b, s);
-        if (ev) MGB_CUDA(cudaEventRecord(ev[0], s));
-        rep_col3(g, b, n, s);
-        if (ev) MGB_CUDA(cudaEventRecord(ev[1], s));
-        rep_row_inv3(g, b, s);
-        if (ev) MGB_CUDA(cudaEventRecord(ev[2], s));
+        const LoopArgs a{rep_desc(b, g, n), nullptr, 1};
+        const LoopSizes z{n, b.Nmax, b.Mmax, b.Mp3max, b.ni};
+        rep_row_fwd3(a, z, s);
+        rep_col3(a, z, s);
+        rep_row_inv3(a, z, s);
         return;
     }
     const size_t smem = fft_smem(b.Mmax);
@@ -511,16 +527,13 @@ void rep_convolve(GridDesc* g, RepBuffers& b, int64_t n, cudaStream_t s, cudaEve
     row_fwd_kernel<<<fft_blocks(pairs), kFftThreads, smem, s>>>(g, b.W.as<float4>(), b.Nmax, b.WhT.as<float2>(),
                                                                 b.Npmax, b.Mhmax, b.tw.as<float2>());
     MGB_LAUNCH_CHECK();
-    if (ev) MGB_CUDA(cudaEventRecord(ev[0], s));
     col_kernel<<<fft_blocks(b.Mhmax), kFftThreads, smem, s>>>(g, b.WhT.as<float2>(), b.PhT.as<float2>(), b.Npmax,
                                                               b.Mhmax, b.Kt.as<float>(), b.Mmax, b.tw.as<float2>(),
                                                               b.zpart.as<double>(), n);
     MGB_LAUNCH_CHECK();
-    if (ev) MGB_CUDA(cudaEventRecord(ev[1], s));
     row_inv_kernel<<<fft_blocks(pairs), kFftThreads, smem, s>>>(g, b.PhT.as<float2>(), b.Npmax, b.Mhmax,
                                                                 b.phi.as<float>(), b.Nmax, b.tw.as<float2>());
     MGB_LAUNCH_CHECK();
-    if (ev) MGB_CUDA(cudaEventRecord(ev[2], s));
 }
 
 void rep_twiddles(GridDesc* g, RepBuffers& b, cudaStream_t s, bool force) {
@@ -536,15 +549,12 @@ void rep_prepare_device_spectra(RepBuffers& b) {
     ensure_fft_attrs();
 }
 
-void rep_update_spectra(GridDesc* g, RepBuffers& b, float dof, cudaStream_t s) {
-    const int Pa = b.Mmax / 2 + 1;
-    require(b.Rt.p != nullptr, "rep_prepare_device_spectra must run first");
-    const size_t smem = fft_smem(b.Mmax);
-    spec_rows_kernel<<<fft_blocks(Pa), kFftThreads, smem, s>>>(g, b.Rt.as<float2>(), Pa, b.Mhmax, b.tw.as<float2>(),
-                                                                b.ni, (double)dof);
+void rep_update_spectra(const LoopArgs& a, int Mmax, cudaStream_t s) {
+    const size_t smem = fft_smem(Mmax);
+    const int bx = std::max(1, ceil_div(2 * kNumSMs, a.count));
+    spec_rows_kernel<<<dim3(std::min(bx, Mmax / 2 + 1), a.count), kFftThreads, smem, s>>>(a);
     MGB_LAUNCH_CHECK();
-    spec_cols_kernel<<<fft_blocks(2 * b.Mhmax), kFftThreads, smem, s>>>(g, b.Rt.as<float2>(), Pa, b.Mhmax,
-                                                                         b.Kt.as<float>(), b.Mmax, b.tw.as<float2>());
+    spec_cols_kernel<<<dim3(std::min(bx, Mmax + 2), a.count), kFftThreads, smem, s>>>(a);
     MGB_LAUNCH_CHECK();
 }
 

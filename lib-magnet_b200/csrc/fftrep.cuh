@@ -5,6 +5,8 @@
 //   W    float4 [N][N]        spread charges (1, x, y, -) per node, interleaved; zeroed by the forward rows
 //   WhT  float2 [3][Mh][Np]   row spectra, transposed (node row index contiguous) for the column pass
 //   PhT  float2 [4][Mh][Np]   products after the inverse column transforms, same layout
+//        The in-place engine holds channel 0 in WhT[0] / PhT[1] by frequency, and x W + i y W, one complex field, in
+//        the M rows from WhT[1] / PhT[2] on by position (the order its stages leave)
 //   phi  float  [4][N][N]     potentials per channel (planar)
 //   Kt   float  [2][Mh][M]    kernel spectra K1h, K2h transposed (k1 contiguous)
 //   Rt   float2 [2][Mh][M/2+1] row spectra of the two kernels (spectrum generation only)
@@ -15,6 +17,8 @@
 #include "common.cuh"
 
 namespace mgb {
+
+namespace fft3 { struct Plan; }
 
 struct GridDesc {
     float xmin, ymin, width, inv_width;
@@ -35,12 +39,48 @@ struct GridDesc {
 
 struct RepBuffers {
     int Nmax = 0, Mmax = 0, Mhmax = 0, Npmax = 0, ni = 3;
-    DevBuf W, WhT, PhT, phi, Kt, Rt, tw, zpart, fft_len_table, bbox_part, mean_part;
-    int max_bbox_blocks = 0;
+    DevBuf W, WhT, PhT, phi, Kt, Rt, tw, zpart, fft_len_table;
     DevBuf plans3;            // in-place engine (fft3.cuh) plans, indexed by M
     int Mp3max = 0;           // its largest padded length up to Mmax
     bool use3 = false;        // the in-place column pass (fftrep3.cu) runs every length these buffers see
     void alloc(int Nmax_, int Mmax_, int ni_);
+};
+
+// What the in-place engine and the t-SNE loop's kernels read of one layout (device addresses, sizes, schedule)
+struct TsneSched {
+    int early_iter;
+    float early_exag, exag, mom0, mom1, lr, inv_dof;
+    double box_width;
+    int min_boxes, max_boxes, ni;
+};
+
+struct LoopDesc {
+    GridDesc* g;
+    float4* W; float2* WhT; float2* PhT; float* phi; float* Kt; float2* Rt; float2* tw;
+    const fft3::Plan* plans; double* zpart; const int* fft_len;
+    int Nmax, Npmax, Mhmax, Mmax;
+    int64_t n;
+    // the loop only
+    float2* Ycur; float2* Ynext; float2* U; float2* G;
+    const int32_t* ip; const int32_t* ix; const float* P;
+    float4* box_part; double2* mean_part;
+    TsneSched sch;
+    double dof;
+};
+
+// the layouts of one launch: `one`, or `count` of them in device memory (at most kMaxLoops)
+constexpr int kMaxLoops = 1024;
+struct LoopArgs {
+    LoopDesc one;
+    const LoopDesc* many;
+    int count;
+};
+
+// the largest of a launch's layouts
+struct LoopSizes {
+    int64_t n;            // points
+    int Nmax, Mmax, Mp;   // grid side, FFT side, padded FFT length
+    int ni;
 };
 
 // host-side next_fast_len(target, real=True) of scipy: smallest 5-smooth integer >= target
@@ -53,8 +93,7 @@ void rep_set_grid_host(GridDesc* g_dev, float xmin, float ymin, float width, int
                        cudaStream_t s);
 void rep_spread(const float2* Y, int64_t n, GridDesc* g, RepBuffers& b, cudaStream_t s);
 void rep_prepare_device_spectra(RepBuffers& b);   // before capture: scratch of the spectrum generation
-void rep_update_spectra(GridDesc* g, RepBuffers& b, float dof, cudaStream_t s);
-void rep_convolve(GridDesc* g, RepBuffers& b, int64_t n, cudaStream_t s, cudaEvent_t* ev = nullptr);
+void rep_convolve(GridDesc* g, RepBuffers& b, int64_t n, cudaStream_t s);
 void rep_gather_forces(const float2* Y, int64_t n, GridDesc* g, RepBuffers& b, float2* F, cudaStream_t s);
 void rep_set_spectra_from_host_layout(RepBuffers& b, const float* K1h_dev, const float* K2h_dev, int M,
                                       cudaStream_t s);
@@ -65,16 +104,14 @@ int noalloc_max_fft_side();
 void fftconv_compute_noalloc(const float* K1h, const float* K2h, int M, int n_interp, const float* Y, int64_t n,
                              float xmin, float ymin, float width, int n_boxes, float* sumQ, float* F);
 
-// in-place engine (fftrep3.cu)
+// in-place engine (fftrep3.cu): the three transforms over every layout of the launch
 void fft3_build_plans(DevBuf& table, int Mmax, int& Mp_max);
-int col3_blocks(int Mp_max);
-void fft3_prepare(int Mp_max);
-void rep_col3(GridDesc* g, RepBuffers& b, int64_t n, cudaStream_t s);
-void rep_row_fwd3(GridDesc* g, RepBuffers& b, cudaStream_t s);
-void rep_row_inv3(GridDesc* g, RepBuffers& b, cudaStream_t s);
-
-
-// the whole t-SNE iteration pieces (tsne.cu)
-struct TsneDev;
+void fft3_prepare(int Mp_max);   // shared-memory limits, before any capture
+void rep_row_fwd3(const LoopArgs& a, const LoopSizes& z, cudaStream_t s);
+void rep_col3(const LoopArgs& a, const LoopSizes& z, cudaStream_t s);
+void rep_row_inv3(const LoopArgs& a, const LoopSizes& z, cudaStream_t s);
+// kernel spectra of the layouts whose grid changed
+void rep_update_spectra(const LoopArgs& a, int Mmax, cudaStream_t s);
+LoopDesc rep_desc(RepBuffers& b, GridDesc* g, int64_t n);   // the FFT fields
 
 }  // namespace mgb

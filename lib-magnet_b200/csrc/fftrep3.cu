@@ -1,15 +1,23 @@
-// Column pass of the FFT repulsion on the in-place engine (fft3.cuh): src/fftconv.cpp:146-186 (forward column
-// transforms, products with the real kernel spectra, inverse column transforms) and the FP64 Z of :226-229.
+// The FFT repulsion's three transforms on the in-place engine (fft3.cuh): forward rows, columns with the kernel
+// products, inverse rows (src/fftconv.cpp:124-199), and the FP64 Z of :226-229.
 //
-// One work item per (column k of the row half-spectra, channel c), persistent blocks, one shared-memory buffer
-// per block (three blocks per SM, so that one block's barriers overlap the others' stages):
-//   channels 1 and 2 (x W, y W): forward, times K2, inverse, into outputs 2 and 3;
-//   channel 0 (W): forward; sum K1 |W0h|^2 for Z from its spectrum, and its product with K2 into output 1. The
-//   reference's potential K1 x W0 (output 0) is never formed: Z comes from the spectrum (Parseval) and the gather
-//   reads the potentials 1-3 only.
-// The first forward stage reads the live rows (g < N) of WhT from global memory, the last inverse stage writes
-// the live rows of PhT, so a column costs 2 (S - 1) shared-memory passes per transform and no reordering pass.
+// The three real charge fields run as two transforms. x W and y W are packed as one complex field x W + i y W: its
+// column products with the real kernel spectrum give phi_2 + i phi_3, so nothing is ever separated and its spectrum
+// stays in the order the stages leave (row position p of the transposed buffer holds frequency freq_of_pos(p)). The
+// charge field W needs its own spectrum for Z; two of its rows share a transform, separated into half spectra after
+// the forward rows and rebuilt before the inverse ones.
+//
+// Work items: rows by pairs (x W + i y W) or fours (W), columns by position (x W + i y W) or frequency (W), one per
+// block at a time. The items of all layouts of a launch are one list, dealt over the resident blocks.
+//
+//   columns: the first forward stage reads the live rows (g < N) from global memory, the last inverse stage writes the
+//   live rows, so a column costs 2 (S - 1) shared-memory passes per transform and no reordering pass.
 // Output convention as the one-radix engine: PhT = unnormalised inverse (M x the circular convolution).
+//
+// Bound by the scattered 16 and 32 byte transposed accesses (rows) and by the latency of the stages at 4 to 6 warps per
+// scheduler (columns). Packing the fields took a third of the transforms' work off the columns and the separation off
+// the rows; M = 4320: forward rows 133 to 131 us, columns 255 to 231, inverse rows 166 to 153; M = 2400: 76 to 50, 96 to
+// 87, 89 to 59.
 #include "fftrep.cuh"
 #include "fft3.cuh"
 #include <vector>
@@ -19,49 +27,144 @@ namespace mgb {
 
 namespace {
 
-constexpr int kColThreads = 256;
+constexpr int kColThreads = 192;
+constexpr int kRowThreads = 256;
+// Blocks per SM the registers are capped for (80 a thread in the columns, 128 in the rows). A loop's buffers are sized
+// for its largest length (M = 6000: 50 KB a column, 100 KB a row block), so more row blocks would not fit beside each
+// other; at M = 4320 3 x 256 and 4 x 128 threads took 142 and 147 us forward, 169 and 208 us inverse, against 127 and
+// 157 us.
+constexpr int kColBlocks = 4;
+constexpr int kRowBlocks = 2;
 
-// transform t of a column pass reads / writes column k of channel a (t = 0) or b (t = 1)
-struct ColLoad {
-    const float2* a;
-    const float2* b;
-    __device__ __forceinline__ float2 operator()(int t, int n) const { return (t ? b : a)[n]; }
-};
-struct ColStore {
-    float2* a;
-    float2* b;
-    __device__ __forceinline__ void operator()(int t, int n, float2 v) const { (t ? b : a)[n] = v; }
+// ---------------------------------------------------------------------------------------------- items
+// the launch's items: layout l holds items [first[l], first[l + 1])
+struct Items {
+    int first[kMaxLoops + 1];
 };
 
-// last forward stage, product with one real kernel spectrum, first inverse stage (in place), on nbuf buffers
-template <int R>
-__device__ __noinline__ void middle1(const fft3::Plan& p, float2* __restrict__ A, float2* __restrict__ B, int nbuf,
-                                     const float* __restrict__ K) {
-    const int pb = p.padR ? R + 1 : R;
-    const int nb = p.M / R;
-    for (int i = threadIdx.x; i < nb * nbuf; i += blockDim.x) {
-        const int t = i >= nb ? 1 : 0;
-        const int b = i - t * nb;
-        float2* buf = t ? B : A;
-        const int base = b * pb;
-        float2 v[R];
+// items_of(N, M) per layout; called by the whole block
+template <bool MANY, class F>
+__device__ __forceinline__ void list_items(const LoopArgs& a, Items& it, F items_of) {
+    if (!MANY) {
+        if (threadIdx.x == 0) {
+            it.first[0] = 0;
+            it.first[1] = items_of(a.one.g->N, a.one.g->M);
+        }
+        __syncthreads();
+        return;
+    }
+    for (int l = threadIdx.x; l < a.count; l += blockDim.x) {
+        const GridDesc* g = a.many[l].g;
+        it.first[l + 1] = items_of(g->N, g->M);
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {   // running sums: 32 runs of consecutive layouts
+        const int per = (a.count + 31) / 32, b = threadIdx.x * per, e = min(a.count, b + per);
+        int run = 0;
+        for (int l = b; l < e; ++l) run += it.first[l + 1];
+        int x = run;
 #pragma unroll
-        for (int r = 0; r < R; ++r) v[r] = buf[base + r];
-        fft3::dft_fwd<R>(v);
-        const int fb = fft3::base_freq(p, b);
-#pragma unroll
-        for (int q = 0; q < R; ++q) v[q] = fft::cscale(v[q], __ldg(&K[fb + nb * q]));
-        fft3::dft_inv<R>(v);
-#pragma unroll
-        for (int r = 0; r < R; ++r) buf[base + r] = v[r];
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if ((int)threadIdx.x >= o) x += y;
+        }
+        int acc = x - run;
+        for (int l = b; l < e; ++l) { acc += it.first[l + 1]; it.first[l + 1] = acc; }
+        if (threadIdx.x == 0) it.first[0] = 0;
+    }
+    __syncthreads();
+}
+
+// the layout of an item
+__device__ __forceinline__ int layout_of(const Items& it, int count, int item) {
+    int lo = 0, hi = count;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (it.first[mid] <= item) lo = mid; else hi = mid;
+    }
+    return lo;
+}
+
+// The descriptor of an item's layout: the launch's own (constant operands), or with several layouts a copy in shared
+// memory (held in registers, its pointers were spilled around every stage).
+template <bool MANY>
+__device__ __forceinline__ const LoopDesc& desc_of(const LoopArgs& a, const Items& items, int at, int& item, int& have,
+                                                   LoopDesc& held) {
+    if constexpr (!MANY) {
+        item = at;
+        return a.one;
+    } else {
+        const int l = layout_of(items, a.count, at);
+        item = at - items.first[l];
+        if (l != have) {   // (a barrier has ended the item before)
+            for (int w = threadIdx.x; w < (int)(sizeof(LoopDesc) / sizeof(int)); w += blockDim.x)
+                reinterpret_cast<int*>(&held)[w] = reinterpret_cast<const int*>(a.many + l)[w];
+            __syncthreads();
+            have = l;
+        }
+        return held;
     }
 }
 
-// channel 0: the last forward stage, this thread's share of sum K1 |X|^2 (for Z), the product with K2 and the
+// the block's copy of the plan of its item
+__device__ __forceinline__ void load_plan(const fft3::Plan* plans, int M, fft3::Plan& p, int& have) {
+    if (have != M) {
+        for (int w = threadIdx.x; w < (int)(sizeof(fft3::Plan) / sizeof(int)); w += blockDim.x)
+            reinterpret_cast<int*>(&p)[w] = reinterpret_cast<const int*>(plans + M)[w];
+        __syncthreads();
+        have = M;
+    }
+}
+
+// ---------------------------------------------------------------------------------------------- columns
+// element n of a column at a
+struct ColLoad {
+    const float2* a;
+    __device__ __forceinline__ float2 operator()(int, int n) const { return a[n]; }
+};
+struct ColStore {
+    float2* a;
+    __device__ __forceinline__ void operator()(int, int n, float2 v) const { a[n] = v; }
+};
+
+// A real kernel spectrum along a column. Frequencies k2 past M / 2 read the half spectrum mirrored (kMirror,
+// K(k1, k2) = K(-k1, -k2)); in the complex field's columns 0 and M / 2 the two halves are averaged (kMean), which is
+// what dropping the imaginary parts of those columns does to a real field.
+constexpr int kPlain = 0, kMirror = 1, kMean = 2;
+
+// last forward stage, product with one real kernel spectrum, first inverse stage (in place)
+template <int R>
+__device__ __noinline__ void middle1(const fft3::Plan& p, const float* __restrict__ K, int mode) {
+    float2* const A = fft3::buffers();
+    const int pb = p.padR ? R + 1 : R;
+    const int nb = p.M / R;
+    for (int b = threadIdx.x; b < nb; b += blockDim.x) {
+        const int base = b * pb;
+        float2 v[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = A[base + r];
+        fft3::dft_fwd<R>(v);
+        // frequency f of the column, or M - f (0 stays 0): a step from the first, and its end only where f is 0
+        const int fb = fft3::base_freq(p, b);
+        const int f0 = mode == kMirror ? p.M - fb : fb, step = mode == kMirror ? -nb : nb;
+        float kv[R];
+#pragma unroll
+        for (int q = 0; q < R; ++q) kv[q] = __ldg(&K[q == 0 && f0 == p.M ? 0 : f0 + step * q]);
+        if (mode == kMean)
+            for (int q = 0; q < R; ++q) { const int f = fb + nb * q; kv[q] = 0.5f * (kv[q] + __ldg(&K[f ? p.M - f : 0])); }
+#pragma unroll
+        for (int q = 0; q < R; ++q) v[q] = fft::cscale(v[q], kv[q]);
+        fft3::dft_inv<R>(v);
+#pragma unroll
+        for (int r = 0; r < R; ++r) A[base + r] = v[r];
+    }
+}
+
+// the charge field: the last forward stage, this thread's share of sum K1 |X|^2 (for Z), the product with K2 and the
 // first inverse stage (in place in A); returns the share
 template <int R>
-__device__ __noinline__ double middle2(const fft3::Plan& p, float2* __restrict__ A, const float* __restrict__ K1,
-                                       const float* __restrict__ K2) {
+__device__ __noinline__ double middle2(const fft3::Plan& p, const float* __restrict__ K1, const float* __restrict__ K2) {
+    float2* const A = fft3::buffers();
     const int pb = p.padR ? R + 1 : R;
     const int nb = p.M / R;
     double zs = 0.0;
@@ -87,169 +190,192 @@ __device__ __noinline__ double middle2(const fft3::Plan& p, float2* __restrict__
     return zs;
 }
 
-__device__ __forceinline__ double middle2_dispatch(int R, const fft3::Plan& p, float2* A, const float* K1,
-                                                   const float* K2) {
+__device__ __forceinline__ double middle2_dispatch(int R, const fft3::Plan& p, const float* K1, const float* K2) {
     switch (R) {
-        case 2: return middle2<2>(p, A, K1, K2);
-        case 3: return middle2<3>(p, A, K1, K2);
-        case 4: return middle2<4>(p, A, K1, K2);
-        case 5: return middle2<5>(p, A, K1, K2);
-        case 6: return middle2<6>(p, A, K1, K2);
-        case 8: return middle2<8>(p, A, K1, K2);
-        case 9: return middle2<9>(p, A, K1, K2);
-        case 10: return middle2<10>(p, A, K1, K2);
-        case 12: return middle2<12>(p, A, K1, K2);
-        case 15: return middle2<15>(p, A, K1, K2);
-        case 16: return middle2<16>(p, A, K1, K2);
-        case 18: return middle2<18>(p, A, K1, K2);
-        default: return middle2<20>(p, A, K1, K2);
+        case 2: return middle2<2>(p, K1, K2);
+        case 3: return middle2<3>(p, K1, K2);
+        case 4: return middle2<4>(p, K1, K2);
+        case 5: return middle2<5>(p, K1, K2);
+        case 6: return middle2<6>(p, K1, K2);
+        case 8: return middle2<8>(p, K1, K2);
+        case 9: return middle2<9>(p, K1, K2);
+        case 10: return middle2<10>(p, K1, K2);
+        case 12: return middle2<12>(p, K1, K2);
+        case 15: return middle2<15>(p, K1, K2);
+        case 16: return middle2<16>(p, K1, K2);
+        case 18: return middle2<18>(p, K1, K2);
+        default: return middle2<20>(p, K1, K2);
     }
 }
 
-// One (column, channel) per work item, one shared-memory buffer per block: the three channels' convolutions are
-// independent (channel 0 also yields the column's Z share), so a block holds a single transform and the SM
-// holds more blocks to overlap one block's barriers with another's stages.
-constexpr int kColBlocks = 3;   // 3 x 80 registers x 256 threads; 3 buffers of M = 6000 fit the SM
-
-__global__ void __launch_bounds__(kColThreads, kColBlocks) col3_kernel(GridDesc* __restrict__ gd,
-                                                              const fft3::Plan* __restrict__ plans,
-                                                              const float2* __restrict__ WhT, float2* __restrict__ PhT,
-                                                              int Np, int Mhmax, const float* __restrict__ Kt, int Mmax,
-                                                              const float2* __restrict__ tw,
-                                                              double* __restrict__ zpart, int64_t n_points) {
-    extern __shared__ float2 sm[];
-    __shared__ fft3::Plan p;
-    __shared__ double red[kColThreads / 32];
-    __shared__ int is_last;
-    const int N = gd->N, M = gd->M, Mh = gd->Mh;
-    if (threadIdx.x == 0) p = plans[M];
+// FP64 sum over the block (in its first thread)
+__device__ __forceinline__ double block_sum(double x, double* red) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = x;
     __syncthreads();
-    float2* A = sm;
-    const int S = p.S;
-    const int R0 = p.st[0].R, RS = p.st[S - 1].R;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int item = blockIdx.x; item < 3 * Mh; item += gridDim.x) {
-        // channel 0 first for every column, so that the Z shares are ready early
-        const int c = item < Mh ? 0 : (item < 2 * Mh ? 1 : 2);
-        const int k = item - c * Mh;
-        const float2* src = WhT + ((size_t)c * Mhmax + k) * Np;
-        float2* dst = PhT + ((size_t)(c + 1) * Mhmax + k) * Np;
-        const float* K1 = Kt + (size_t)k * Mmax;
-        const float* K2 = Kt + ((size_t)Mhmax + k) * Mmax;
-        MGB_FFT3_RADIX_DISPATCH(R0, fft3::dif_first, p, A, A, 1, ColLoad{src, src}, N, tw);
+    double s = 0.0;
+    if (threadIdx.x == 0)
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[w];
+    return s;
+}
+
+template <bool MANY>
+__global__ void __launch_bounds__(kColThreads, kColBlocks) col3_kernel(const __grid_constant__ LoopArgs a) {
+    __shared__ Items items;
+    __shared__ fft3::Plan p;
+    __shared__ LoopDesc held;
+    __shared__ double red[kColThreads / 32];
+    __shared__ int last;
+    // the charge field's columns first, so that the Z shares are ready early
+    list_items<MANY>(a, items, [](int, int M) { return M / 2 + 1 + M; });
+    int have = -1, have_l = -1;
+    int N = MANY ? 0 : a.one.g->N, M = MANY ? 0 : a.one.g->M;
+    const int total = items.first[MANY ? a.count : 1];
+    for (int at = blockIdx.x; at < total; at += gridDim.x) {
+        int item;
+        const LoopDesc& L = desc_of<MANY>(a, items, at, item, have_l, held);
+        if (MANY) { N = L.g->N; M = L.g->M; }
+        const int Mh = M / 2 + 1;
+        load_plan(L.plans, M, p, have);
+        const int S = p.S, R0 = p.st[0].R, RS = p.st[S - 1].R;
+        const bool charge = item < Mh;
+        const int row = charge ? item : item - Mh;                     // row of the transposed buffers
+        const int f2 = charge ? row : fft3::freq_of_pos(p, row);       // the column's frequency
+        const int k = f2 < Mh ? f2 : M - f2;
+        const int mode = charge ? kPlain : (f2 >= Mh ? kMirror : (k == 0 || 2 * k == M ? kMean : kPlain));
+        const float2* src = L.WhT + ((size_t)(charge ? 0 : L.Mhmax) + row) * L.Npmax;
+        float2* dst = L.PhT + ((size_t)(charge ? L.Mhmax : 2 * L.Mhmax) + row) * L.Npmax;
+        const float* K2 = L.Kt + ((size_t)L.Mhmax + k) * L.Mmax;
+        const float2* tw = L.tw;
+        MGB_FFT3_RADIX_DISPATCH(R0, fft3::dif_first, p, 0, 0, 1, ColLoad{src}, N, tw);
         __syncthreads();
         for (int s = 1; s < S - 1; ++s) {
-            MGB_FFT3_RADIX_DISPATCH(p.st[s].R, fft3::dif_mid, p, s, A, A, 1, tw);
+            MGB_FFT3_RADIX_DISPATCH(p.st[s].R, fft3::dif_mid, p, s, 0, 0, 1, tw);
             __syncthreads();
         }
-        if (c == 0) {
-            double zs = middle2_dispatch(RS, p, A, K1, K2);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) zs += __shfl_xor_sync(0xffffffffu, zs, o);
-            if (lane == 0) red[warp] = zs;
-            __syncthreads();
+        if (charge) {
+            const double z = block_sum(middle2_dispatch(RS, p, L.Kt + (size_t)k * L.Mmax, K2), red);
             if (threadIdx.x == 0) {
-                double t = 0.0;
-                for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
                 const bool single = (k == 0) || ((M & 1) == 0 && k == M / 2);
-                zpart[k] = single ? t : 2.0 * t;
+                L.zpart[k] = single ? z : 2.0 * z;
+                __threadfence();
+                last = atomicAdd(&L.g->counter, 1u) == (unsigned)(Mh - 1);
+            }
+            __syncthreads();
+            if (last) {
+                // the block that finishes the layout's last share: Z = sum of the shares / M^2 - n
+                __threadfence();
+                double x = 0.0;
+                for (int q = threadIdx.x; q < Mh; q += blockDim.x) x += __ldcg(&L.zpart[q]);
+                x = block_sum(x, red);
+                if (threadIdx.x == 0) {
+                    const double sumQ = x / ((double)M * (double)M) - (double)L.n;
+                    L.g->sumQ = sumQ;
+                    const float sf = (float)sumQ;
+                    L.g->sumQ_f = sf;
+                    L.g->inv_sumQ = (float)(1.0 / fmax((double)sf, 1e-12));
+                    L.g->counter = 0u;
+                }
             }
         } else {
-            MGB_FFT3_RADIX_DISPATCH(RS, middle1, p, A, A, 1, K2);
+            MGB_FFT3_RADIX_DISPATCH(RS, middle1, p, K2, mode);
             __syncthreads();
         }
         for (int s = S - 2; s >= 1; --s) {
-            MGB_FFT3_RADIX_DISPATCH(p.st[s].R, fft3::dit_mid, p, s, A, A, 1, tw);
+            MGB_FFT3_RADIX_DISPATCH(p.st[s].R, fft3::dit_mid, p, s, 0, 0, 1, tw);
             __syncthreads();
         }
-        MGB_FFT3_RADIX_DISPATCH(R0, fft3::dit_last, p, A, A, 1, ColStore{dst, dst}, N, tw);
+        MGB_FFT3_RADIX_DISPATCH(R0, fft3::dit_last, p, 0, 0, 1, ColStore{dst}, N, tw);
         __syncthreads();
-    }
-    // last block: Z = sum of the partials / M^2 - n
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) is_last = (atomicAdd(&gd->counter, 1u) == gridDim.x - 1);
-    __syncthreads();
-    if (!is_last) return;
-    __threadfence();
-    double t = 0.0;
-    for (int k = threadIdx.x; k < Mh; k += blockDim.x) t += __ldcg(&zpart[k]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if (lane == 0) red[warp] = t;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double s = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[w];
-        const double sumQ = s / ((double)M * (double)M) - (double)n_points;
-        gd->sumQ = sumQ;
-        const float sf = (float)sumQ;
-        gd->sumQ_f = sf;
-        gd->inv_sumQ = (float)(1.0 / fmax((double)sf, 1e-12));
-        gd->counter = 0u;
     }
 }
 
 // ---------------------------------------------------------------------------------------------- rows
-// A block owns 4 grid rows g0..g0+3 (src/fftconv.cpp:129-143 forward, :188-198 inverse). Rows are packed two per
-// complex sequence (z = w_g + i w_{g+1}); buffer A holds the pair (g0, g0+1), buffer B the pair (g0+2, g0+3), so
-// the transposed spectra of the 4 rows are read and written as 32 contiguous bytes per frequency.
-constexpr int kRowThreads = 256;
+// Two buffers per block. Items of a layout: the charge field's rows by fours (first, they are the longer ones), then the
+// complex field's rows by pairs. The transposed spectra are read and written 16 (a pair of complex rows) or 32 (four
+// rows' half spectra) contiguous bytes per frequency.
 
-__device__ __forceinline__ float chan(const float4& v, int c) { return c == 0 ? v.x : (c == 1 ? v.y : v.z); }
-
-// channel c of rows g0..g0+3 of the charge grid (rows at or past N read as zero)
-struct RowLoad {
+// rows g0 + 2t and g0 + 2t + 1 of the charges, packed as one complex row (rows at or past N read as zero)
+struct ChargeLoad {
     const float4* W;
-    int pitch, g0, N, c;
+    int pitch, g0, N;
     __device__ __forceinline__ float2 operator()(int t, int n) const {
         const int ga = g0 + 2 * t, gb = ga + 1;
-        const float x = ga < N ? chan(W[(size_t)ga * pitch + n], c) : 0.f;
-        const float y = gb < N ? chan(W[(size_t)gb * pitch + n], c) : 0.f;
+        const float x = ga < N ? W[(size_t)ga * pitch + n].x : 0.f;
+        const float y = gb < N ? W[(size_t)gb * pitch + n].x : 0.f;
         return make_float2(x, y);
     }
 };
-
-// potential channel c of rows g0..g0+3: Re to row g0 + 2t, Im to row g0 + 2t + 1, scaled by 1 / M^2
-struct PhiStore {
-    float* phi;
-    size_t plane;
-    int pitch, g0, N, c;
-    float scale;
-    __device__ __forceinline__ void operator()(int t, int n, float2 v) const {
-        const int ga = g0 + 2 * t, gb = ga + 1;
-        float* base = phi + (size_t)c * plane + n;
-        if (ga < N) base[(size_t)ga * pitch] = v.x * scale;
-        if (gb < N) base[(size_t)gb * pitch] = v.y * scale;
+// row g0 + t of the complex field
+struct FieldLoad {
+    const float4* W;
+    int pitch, g0;
+    __device__ __forceinline__ float2 operator()(int t, int n) const {
+        const float4 v = W[(size_t)(g0 + t) * pitch + n];
+        return make_float2(v.y, v.z);
     }
 };
 
-// Forward row transforms of the 3 charge channels, separated into the half spectra of the 4 rows and written
-// transposed (WhT[c][k][g]); the consumed rows of W are zeroed for the next spread.
-__global__ void __launch_bounds__(kRowThreads, 2) row_fwd3_kernel(const GridDesc* __restrict__ gd,
-                                                                  const fft3::Plan* __restrict__ plans,
-                                                                  float4* __restrict__ W, int pitchW,
-                                                                  float2* __restrict__ WhT, int Np, int Mhmax,
-                                                                  const float2* __restrict__ tw) {
-    extern __shared__ float2 sm[];
+// potential 1 of rows g0 + 2t (Re) and g0 + 2t + 1 (Im), scaled by 1 / M^2
+struct ChargeStore {
+    float* phi;
+    int pitch, g0, N;
+    float scale;
+    __device__ __forceinline__ void operator()(int t, int n, float2 v) const {
+        const int ga = g0 + 2 * t, gb = ga + 1;
+        if (ga < N) phi[(size_t)ga * pitch + n] = v.x * scale;
+        if (gb < N) phi[(size_t)gb * pitch + n] = v.y * scale;
+    }
+};
+// potentials 2 (Re) and 3 (Im) of row g0 + t
+struct FieldStore {
+    float* phi2;
+    float* phi3;
+    int pitch, g0;
+    float scale;
+    __device__ __forceinline__ void operator()(int t, int n, float2 v) const {
+        const size_t at = (size_t)(g0 + t) * pitch + n;
+        phi2[at] = v.x * scale;
+        phi3[at] = v.y * scale;
+    }
+};
+
+__device__ __forceinline__ int row_items(int N) { return (N + 3) / 4 + (N + 1) / 2; }
+
+template <bool MANY>
+__global__ void __launch_bounds__(kRowThreads, kRowBlocks) row_fwd3_kernel(const __grid_constant__ LoopArgs a) {
+    __shared__ Items items;
     __shared__ fft3::Plan p;
-    const int N = gd->N, M = gd->M, Mh = gd->Mh;
-    if (threadIdx.x == 0) p = plans[M];
-    __syncthreads();
-    float2* A = sm;
-    float2* B = sm + p.Mp;
-    const int S = p.S;
-    const int groups = (N + 3) / 4;
-    for (int grp = blockIdx.x; grp < groups; grp += gridDim.x) {
-        const int g0 = 4 * grp;
-        const int nbuf = g0 + 2 < N ? 2 : 1;
-        for (int c = 0; c < 3; ++c) {
-            MGB_FFT3_RADIX_DISPATCH(p.st[0].R, fft3::dif_first, p, A, B, nbuf, RowLoad{W, pitchW, g0, N, c}, N, tw);
+    __shared__ LoopDesc held;
+    list_items<MANY>(a, items, [](int N, int) { return row_items(N); });
+    int have = -1, have_l = -1;
+    int N = MANY ? 0 : a.one.g->N, M = MANY ? 0 : a.one.g->M;
+    const int total = items.first[MANY ? a.count : 1];
+    float2* const A = fft3::buffers();
+    for (int at = blockIdx.x; at < total; at += gridDim.x) {
+        int item;
+        const LoopDesc& L = desc_of<MANY>(a, items, at, item, have_l, held);
+        if (MANY) { N = L.g->N; M = L.g->M; }
+        const int Mh = M / 2 + 1;
+        load_plan(L.plans, M, p, have);
+        float2* const B = A + p.Mp;
+        const int fours = (N + 3) / 4;
+        const bool charge = item < fours;
+        const int g0 = charge ? 4 * item : 2 * (item - fours);
+        const int nbuf = g0 + (charge ? 2 : 1) < N ? 2 : 1;
+        const float2* tw = L.tw;
+        if (charge) {
+            MGB_FFT3_RADIX_DISPATCH(p.st[0].R, fft3::dif_first, p, 0, p.Mp, nbuf, ChargeLoad{L.W, L.Nmax, g0, N}, N, tw);
+        } else {
+            MGB_FFT3_RADIX_DISPATCH(p.st[0].R, fft3::dif_first, p, 0, p.Mp, nbuf, FieldLoad{L.W, L.Nmax, g0}, N, tw);
+        }
+        __syncthreads();
+        for (int s = 1; s < p.S; ++s) {
+            MGB_FFT3_RADIX_DISPATCH(p.st[s].R, fft3::dif_mid, p, s, 0, p.Mp, nbuf, tw);
             __syncthreads();
-            for (int s = 1; s < S; ++s) {
-                MGB_FFT3_RADIX_DISPATCH(p.st[s].R, fft3::dif_mid, p, s, A, B, nbuf, tw);
-                __syncthreads();
-            }
+        }
+        if (charge) {
             // rows a, b of a pair from Z_k and Z_{-k}: (Z_k + conj Z_{-k}) / 2 and (Z_k - conj Z_{-k}) / 2i; walked in
             // position order (consecutive threads read consecutive positions), frequencies past M/2 skipped
             for (int pos = threadIdx.x; pos < M; pos += blockDim.x) {
@@ -257,79 +383,100 @@ __global__ void __launch_bounds__(kRowThreads, 2) row_fwd3_kernel(const GridDesc
                 if (k >= Mh) continue;
                 const int pk = p.padR ? pos + fft3::udiv(pos, p.mpad) : pos;
                 const int pm = fft3::pos_of_freq(p, k == 0 ? 0 : M - k);
-                float2* dst = WhT + ((size_t)c * Mhmax + k) * Np + g0;
-                for (int t = 0; t < nbuf; ++t) {
-                    const float2* buf = t ? B : A;
+                float2* dst = L.WhT + (size_t)k * L.Npmax + g0;
+                for (int q = 0; q < nbuf; ++q) {
+                    const float2* buf = q ? B : A;
                     const float2 zk = buf[pk], zm = buf[pm];
-                    reinterpret_cast<float4*>(dst)[t] = make_float4(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y),
+                    reinterpret_cast<float4*>(dst)[q] = make_float4(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y),
                                                                     0.5f * (zk.y + zm.y), -0.5f * (zk.x - zm.x));
                 }
             }
-            __syncthreads();
+        } else {
+            float2* dst = L.WhT + (size_t)L.Mhmax * L.Npmax + g0;
+#pragma unroll 4
+            for (int pos = threadIdx.x; pos < M; pos += blockDim.x) {
+                const int pk = p.padR ? pos + fft3::udiv(pos, p.mpad) : pos;
+                const float2 va = A[pk], vb = nbuf > 1 ? B[pk] : make_float2(0.f, 0.f);
+                *reinterpret_cast<float4*>(dst + (size_t)pos * L.Npmax) = make_float4(va.x, va.y, vb.x, vb.y);
+            }
         }
-        const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-        const int rows = min(4, N - g0);
-        for (int i = threadIdx.x; i < rows * N; i += blockDim.x) {
-            const int r = i / N, n = i - r * N;
-            W[(size_t)(g0 + r) * pitchW + n] = z4;
-        }
+        __syncthreads();
     }
 }
 
-// Inverse row transforms of the potential channels 1-3: each pair rebuilt from the two half spectra (Hermitian
-// extension, DC and Nyquist imaginary parts dropped as a c2r does) straight into the digit-reversed positions
-// the inverse stages start from, transformed, scaled by 1/M^2 (src/fftconv.cpp:176, 188-198).
-__global__ void __launch_bounds__(kRowThreads, 2) row_inv3_kernel(const GridDesc* __restrict__ gd,
-                                                                  const fft3::Plan* __restrict__ plans,
-                                                                  const float2* __restrict__ PhT, int Np, int Mhmax,
-                                                                  float* __restrict__ phi, int pitchP,
-                                                                  const float2* __restrict__ tw) {
-    extern __shared__ float2 sm[];
+// The inverse rows; the complex field's items also zero their rows of W for the next spread (every forward row has run).
+template <bool MANY>
+__global__ void __launch_bounds__(kRowThreads, kRowBlocks) row_inv3_kernel(const __grid_constant__ LoopArgs a) {
+    __shared__ Items items;
     __shared__ fft3::Plan p;
-    const int N = gd->N, M = gd->M, Mh = gd->Mh;
-    if (threadIdx.x == 0) p = plans[M];
-    __syncthreads();
-    float2* A = sm;
-    float2* B = sm + p.Mp;
-    const int S = p.S;
-    const bool even = (M & 1) == 0;
-    const float scale = 1.f / ((float)M * (float)M);
-    const size_t plane = (size_t)pitchP * pitchP;
-    const int groups = (N + 3) / 4;
-    for (int grp = blockIdx.x; grp < groups; grp += gridDim.x) {
-        const int g0 = 4 * grp;
-        const int nbuf = g0 + 2 < N ? 2 : 1;
-        for (int c = 1; c < 4; ++c) {   // potentials 1-3 (the gather's); plane 0 is not formed
-            // the spectrum enters in position order: consecutive threads write consecutive positions; the loads of
-            // the transposed spectra are one 32-byte sector per frequency in either order
+    __shared__ LoopDesc held;
+    list_items<MANY>(a, items, [](int N, int) { return row_items(N); });
+    int have = -1, have_l = -1;
+    int N = MANY ? 0 : a.one.g->N, M = MANY ? 0 : a.one.g->M;
+    const int total = items.first[MANY ? a.count : 1];
+    float2* const A = fft3::buffers();
+    for (int at = blockIdx.x; at < total; at += gridDim.x) {
+        int item;
+        const LoopDesc& L = desc_of<MANY>(a, items, at, item, have_l, held);
+        if (MANY) { N = L.g->N; M = L.g->M; }
+        const int Mh = M / 2 + 1;
+        load_plan(L.plans, M, p, have);
+        float2* const B = A + p.Mp;
+        const int fours = (N + 3) / 4;
+        const bool charge = item < fours;
+        const int g0 = charge ? 4 * item : 2 * (item - fours);
+        const int nbuf = g0 + (charge ? 2 : 1) < N ? 2 : 1;
+        const float2* tw = L.tw;
+        const float scale = 1.f / ((float)M * (float)M);
+        const size_t plane = (size_t)L.Nmax * L.Nmax;
+        // the spectra enter in position order (consecutive threads write consecutive positions)
+        if (charge) {
+            // the position's frequency from the half spectra of the rows a, b of each pair: a + i b, past M / 2
+            // conj a + i conj b of its mirror (Hermitian extension, DC and Nyquist imaginary parts dropped as a c2r does;
+            // src/fftconv.cpp:176, 188-198)
+            const bool even = (M & 1) == 0;
 #pragma unroll 2
             for (int up = threadIdx.x; up < M; up += blockDim.x) {
                 const int k = fft3::freq_of_pos(p, up);
                 const int kk = k < Mh ? k : M - k;
-                const float4* src = reinterpret_cast<const float4*>(PhT + ((size_t)c * Mhmax + kk) * Np + g0);
+                const float4* src = reinterpret_cast<const float4*>(L.PhT + ((size_t)L.Mhmax + kk) * L.Npmax + g0);
                 const int pos = p.padR ? up + fft3::udiv(up, p.mpad) : up;
-                for (int t = 0; t < nbuf; ++t) {
-                    const float4 v = src[t];
-                    float2 a = make_float2(v.x, v.y), b = make_float2(v.z, v.w);
-                    if (kk == 0 || (even && kk == M / 2)) { a.y = 0.f; b.y = 0.f; }
-                    if (k >= Mh) { a.y = -a.y; b.y = -b.y; }
-                    (t ? B : A)[pos] = make_float2(a.x - b.y, a.y + b.x);   // a + i b
+                for (int q = 0; q < nbuf; ++q) {
+                    const float4 v = src[q];
+                    float2 x = make_float2(v.x, v.y), y = make_float2(v.z, v.w);
+                    if (kk == 0 || (even && kk == M / 2)) { x.y = 0.f; y.y = 0.f; }
+                    if (k >= Mh) { x.y = -x.y; y.y = -y.y; }
+                    (q ? B : A)[pos] = make_float2(x.x - y.y, x.y + y.x);
                 }
             }
-            __syncthreads();
-            for (int s = S - 1; s >= 1; --s) {
-                MGB_FFT3_RADIX_DISPATCH(p.st[s].R, fft3::dit_mid, p, s, A, B, nbuf, tw);
-                __syncthreads();
+        } else {
+            const float2* src = L.PhT + (size_t)2 * L.Mhmax * L.Npmax + g0;
+#pragma unroll 4
+            for (int up = threadIdx.x; up < M; up += blockDim.x) {
+                const float4 v = __ldg(reinterpret_cast<const float4*>(src + (size_t)up * L.Npmax));
+                const int pos = p.padR ? up + fft3::udiv(up, p.mpad) : up;
+                A[pos] = make_float2(v.x, v.y);
+                if (nbuf > 1) B[pos] = make_float2(v.z, v.w);
             }
-            MGB_FFT3_RADIX_DISPATCH(p.st[0].R, fft3::dit_last, p, A, B, nbuf,
-                                    PhiStore{phi, plane, pitchP, g0, N, c, scale}, N, tw);
+            const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int q = 0; q < nbuf; ++q)
+                for (int n = threadIdx.x; n < N; n += blockDim.x) L.W[(size_t)(g0 + q) * L.Nmax + n] = zero;
+        }
+        __syncthreads();
+        for (int s = p.S - 1; s >= 1; --s) {
+            MGB_FFT3_RADIX_DISPATCH(p.st[s].R, fft3::dit_mid, p, s, 0, p.Mp, nbuf, tw);
             __syncthreads();
         }
+        if (charge) {
+            MGB_FFT3_RADIX_DISPATCH(p.st[0].R, fft3::dit_last, p, 0, p.Mp, nbuf,
+                                    ChargeStore{L.phi + plane, L.Nmax, g0, N, scale}, N, tw);
+        } else {
+            MGB_FFT3_RADIX_DISPATCH(p.st[0].R, fft3::dit_last, p, 0, p.Mp, nbuf,
+                                    FieldStore{L.phi + 2 * plane, L.phi + 3 * plane, L.Nmax, g0, scale}, N, tw);
+        }
+        __syncthreads();
     }
 }
-
-size_t col3_smem(int Mp_max) { return (size_t)Mp_max * sizeof(float2); }       // one transform per column block
-size_t row3_smem(int Mp_max) { return (size_t)2 * Mp_max * sizeof(float2); }   // two row pairs per row block
 
 }  // namespace
 
@@ -346,86 +493,64 @@ void fft3_build_plans(DevBuf& table, int Mmax, int& Mp_max) {
     MGB_CUDA(cudaMemcpy(table.p, plans.data(), plans.size() * sizeof(fft3::Plan), cudaMemcpyHostToDevice));
 }
 
-// resident blocks of the column kernel for this buffer size (raises its shared-memory limit once per device)
-int col3_blocks(int Mp_max) {
-    // per thread: host threads may drive layouts side by side
-    static thread_local int cached_dev = -1, cached_mp = -1, cached_blocks = 0;
-    int dev = 0, optin = 0;
-    MGB_CUDA(cudaGetDevice(&dev));
-    if (cached_dev == dev && cached_mp == Mp_max) return cached_blocks;
-    const size_t smem = col3_smem(Mp_max);
-    MGB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    cudaFuncAttributes a;
-    MGB_CUDA(cudaFuncGetAttributes(&a, (const void*)col3_kernel));
-    require(smem + a.sharedSizeBytes <= (size_t)optin, "FFT side too large for the column engine");
-    MGB_CUDA(cudaFuncSetAttribute((const void*)col3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int per_sm = 0;
-    MGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, col3_kernel, kColThreads, smem));
-    cached_dev = dev;
-    cached_mp = Mp_max;
-    cached_blocks = std::max(1, per_sm) * kNumSMs;
-    return cached_blocks;
-}
-
-// resident blocks of a row kernel (raises its shared-memory limit once per device)
-int row3_blocks(const void* fn, int Mp_max) {
-    const size_t smem = row3_smem(Mp_max);
-    int dev = 0, optin = 0;
-    MGB_CUDA(cudaGetDevice(&dev));
-    MGB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    cudaFuncAttributes a;
-    MGB_CUDA(cudaFuncGetAttributes(&a, fn));
-    require(smem + a.sharedSizeBytes <= (size_t)optin, "FFT side too large for the row engine");
-    MGB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int per_sm = 0;
-    MGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kRowThreads, smem));
-    return std::max(1, per_sm) * kNumSMs;
-}
-
 namespace {
-struct RowBlocks {
-    int dev = -1, mp = -1, fwd = 0, inv = 0;
-};
-thread_local RowBlocks g_row_blocks;   // per thread, as the column cache
-}  // namespace
+size_t col3_smem(int Mp) { return (size_t)Mp * sizeof(float2); }       // one transform per column block
+size_t row3_smem(int Mp) { return (size_t)2 * Mp * sizeof(float2); }   // two per row block
 
-// launch sizes of the row kernels (and their shared-memory limits) for this device and buffer size; called when
-// the buffers are sized, before any stream capture
-void fft3_prepare(int Mp_max) {
+// Threads per block by the largest length of the launch: short transforms have few butterflies per stage (12 of length
+// 144), so a batch of small layouts runs more and smaller blocks.
+int threads_for(int Mmax, int full) { return Mmax <= 1536 ? 64 : full; }
+
+// resident blocks of a kernel for a buffer size and block size
+int resident(const void* fn, int threads, size_t smem) {
+    struct Known { const void* fn; int dev, threads, blocks; size_t smem; };
+    static thread_local std::vector<Known> known;   // per thread: host threads may drive layouts side by side
     int dev = 0;
     MGB_CUDA(cudaGetDevice(&dev));
-    col3_blocks(Mp_max);
-    if (g_row_blocks.dev == dev && g_row_blocks.mp == Mp_max) return;
-    g_row_blocks.fwd = row3_blocks((const void*)row_fwd3_kernel, Mp_max);
-    g_row_blocks.inv = row3_blocks((const void*)row_inv3_kernel, Mp_max);
-    g_row_blocks.dev = dev;
-    g_row_blocks.mp = Mp_max;
+    for (const Known& k : known)
+        if (k.fn == fn && k.dev == dev && k.threads == threads && k.smem == smem) return k.blocks;
+    int per_sm = 0;
+    MGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem));
+    if (known.size() >= 64) known.clear();
+    known.push_back(Known{fn, dev, threads, std::max(1, per_sm) * kNumSMs, smem});
+    return known.back().blocks;
 }
 
-void rep_row_fwd3(GridDesc* g, RepBuffers& b, cudaStream_t s) {
-    fft3_prepare(b.Mp3max);
-    const int blocks = std::min(g_row_blocks.fwd, (b.Nmax + 3) / 4);
-    row_fwd3_kernel<<<blocks, kRowThreads, row3_smem(b.Mp3max), s>>>(
-        g, b.plans3.as<fft3::Plan>(), b.W.as<float4>(), b.Nmax, b.WhT.as<float2>(), b.Npmax, b.Mhmax,
-        b.tw.as<float2>());
+template <class K>
+void launch(K one, K many, const LoopArgs& a, int Mmax, int full, size_t smem, int64_t items, cudaStream_t s) {
+    K fn = a.many ? many : one;
+    const int threads = threads_for(Mmax, full);
+    const int blocks = (int)std::min<int64_t>(resident((const void*)fn, threads, smem), std::max<int64_t>(1, a.count * items));
+    fn<<<blocks, threads, smem, s>>>(a);
     MGB_LAUNCH_CHECK();
 }
+}  // namespace
 
-void rep_row_inv3(GridDesc* g, RepBuffers& b, cudaStream_t s) {
-    fft3_prepare(b.Mp3max);
-    const int blocks = std::min(g_row_blocks.inv, (b.Nmax + 3) / 4);
-    row_inv3_kernel<<<blocks, kRowThreads, row3_smem(b.Mp3max), s>>>(
-        g, b.plans3.as<fft3::Plan>(), b.PhT.as<float2>(), b.Npmax, b.Mhmax, b.phi.as<float>(), b.Nmax,
-        b.tw.as<float2>());
-    MGB_LAUNCH_CHECK();
+// raises the kernels' shared-memory limits; called when buffers are sized, before any stream capture
+void fft3_prepare(int Mp_max) {
+    int dev = 0, optin = 0;
+    MGB_CUDA(cudaGetDevice(&dev));
+    static thread_local int done_dev = -1;   // per thread: host threads may drive layouts side by side
+    MGB_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    cudaFuncAttributes f;
+    for (const void* fn : {(const void*)col3_kernel<false>, (const void*)row_fwd3_kernel<false>, (const void*)row_inv3_kernel<false>,
+                           (const void*)col3_kernel<true>, (const void*)row_fwd3_kernel<true>, (const void*)row_inv3_kernel<true>}) {
+        MGB_CUDA(cudaFuncGetAttributes(&f, fn));
+        require(row3_smem(Mp_max) + f.sharedSizeBytes <= (size_t)optin, "FFT side too large for the row engine");
+        if (done_dev != dev)
+            MGB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)f.sharedSizeBytes));
+    }
+    done_dev = dev;
 }
 
-void rep_col3(GridDesc* g, RepBuffers& b, int64_t n, cudaStream_t s) {
-    const int blocks = std::min(col3_blocks(b.Mp3max), 3 * b.Mhmax);
-    col3_kernel<<<blocks, kColThreads, col3_smem(b.Mp3max), s>>>(
-        g, b.plans3.as<fft3::Plan>(), b.WhT.as<float2>(), b.PhT.as<float2>(), b.Npmax, b.Mhmax, b.Kt.as<float>(),
-        b.Mmax, b.tw.as<float2>(), b.zpart.as<double>(), n);
-    MGB_LAUNCH_CHECK();
+void rep_row_fwd3(const LoopArgs& a, const LoopSizes& z, cudaStream_t s) {
+    launch(row_fwd3_kernel<false>, row_fwd3_kernel<true>, a, z.Mmax, kRowThreads, row3_smem(z.Mp), z.Nmax + 1, s);
+}
+void rep_row_inv3(const LoopArgs& a, const LoopSizes& z, cudaStream_t s) {
+    launch(row_inv3_kernel<false>, row_inv3_kernel<true>, a, z.Mmax, kRowThreads, row3_smem(z.Mp), z.Nmax + 1, s);
+}
+void rep_col3(const LoopArgs& a, const LoopSizes& z, cudaStream_t s) {
+    launch(col3_kernel<false>, col3_kernel<true>, a, z.Mmax, kColThreads, col3_smem(z.Mp), 2LL * z.Mmax, s);
 }
 
 }  // namespace mgb

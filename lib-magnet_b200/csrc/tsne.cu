@@ -2,11 +2,13 @@
 //  * standalone kernels, one per reference call: tsne_attraction (src/fftrep.cpp:129-177), tsne_step (:225-266),
 //    tsne_update (:181-220), bbox_2d (:415-434);
 //  * the whole loop of optimize_tsne (magnet/tsne.py:132-214, common path) with every step on the device:
-//      bbox + grid choice (magnet/tsne.py:30-46) -> [twiddles, kernel spectra when the grid changed
-//      (magnet/tsne.py:48-71)] -> spread -> FFT convolution (+ FP64 Z) -> gather fused with the sparse
-//      attraction and the gains/momentum step (+ FP64 mean for the recentring, applied by the next bbox pass).
+//      spread (recentring the positions on the way) and [kernel spectra when the grid changed (magnet/tsne.py:48-71)]
+//      -> FFT convolution (+ FP64 Z) -> gather fused with the sparse attraction and the gains/momentum step, whose last
+//      block takes the FP64 mean for the recentring, the bounding box, the next grid (magnet/tsne.py:30-46) and its
+//      twiddles.
 //    The iteration reads its schedule (exaggeration, momentum) and every size from device memory, so one
-//    captured CUDA graph is replayed for all iterations.
+//    captured CUDA graph is replayed for all iterations; the spectra are a branch of it beside the spread.
+//    Every kernel runs over a list of layouts (one, or a batch): five launches per iteration on the path, however many.
 #include "tsne.cuh"
 #include "interp.cuh"
 #include "graph.cuh"
@@ -204,42 +206,138 @@ __device__ void choose_grid(GridDesc* g, BBox b, const TsneSched& s, const int* 
     g->tw_M = M;
 }
 
-// recentre (Ycur = Ynext - mean) and bounding box; the last block chooses the grid
-__global__ void __launch_bounds__(kThreads) loop_bbox_kernel(const float2* __restrict__ Ynext, float2* __restrict__ Ycur,
-                                                             int64_t n, GridDesc* __restrict__ g, BBox* __restrict__ part,
-                                                             TsneSched s, const int* __restrict__ fft_len) {
+// the twiddles of a new FFT length, exp(-2 pi i m / M) in FP64, rounded once; by the whole block
+__device__ __noinline__ void make_twiddles(float2* __restrict__ tw, int M) {
+    for (int m = threadIdx.x; m < M; m += blockDim.x) {
+        double s, c;
+        sincospi(-2.0 * (double)m / (double)M, &s, &c);
+        tw[m] = make_float2((float)c, (float)s);
+    }
+}
+
+__device__ __forceinline__ BBox ld_box(const float4* p, unsigned b) {
+    const float4 v = __ldcg(p + b);
+    return BBox{v.x, v.y, v.z, v.w};
+}
+__device__ BBox merge_boxes(const float4* part) {
+    BBox t{INFINITY, INFINITY, -INFINITY, -INFINITY};
+    for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) t = bbox_merge(t, ld_box(part, b));
+    return block_bbox(t);
+}
+
+// bounding box of the starting layout; the last block chooses the grid. Layout blockIdx.y.
+__global__ void __launch_bounds__(kThreads) loop_start_kernel(const __grid_constant__ LoopArgs args) {
     __shared__ int is_last;
-    const bool rc = g->recentre != 0;
-    const float mx = g->mean[0], my = g->mean[1];
+    const LoopDesc L = args.many ? args.many[blockIdx.y] : args.one;
     BBox v{INFINITY, INFINITY, -INFINITY, -INFINITY};
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        float2 p = Ynext[i];
-        if (rc) { p.x = __fsub_rn(p.x, mx); p.y = __fsub_rn(p.y, my); }
-        Ycur[i] = p;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < L.n; i += (int64_t)gridDim.x * blockDim.x) {
+        const float2 p = L.Ynext[i];
         v = bbox_merge(v, BBox{p.x, p.y, p.x, p.y});
     }
     v = block_bbox(v);
-    if (threadIdx.x == 0) { part[blockIdx.x] = v; __threadfence(); is_last = atomicAdd(&g->counter2, 1u) == gridDim.x - 1; }
+    if (threadIdx.x == 0) {
+        L.box_part[blockIdx.x] = make_float4(v.x0, v.y0, v.x1, v.y1);
+        __threadfence();
+        is_last = atomicAdd(&L.g->counter2, 1u) == gridDim.x - 1;
+    }
     __syncthreads();
     if (!is_last) return;
     __threadfence();
-    const BBox t = merge_parts(part);
-    if (threadIdx.x != 0) return;
-    choose_grid(g, t, s, fft_len);
-    g->counter2 = 0u;
+    const BBox t = merge_boxes(L.box_part);
+    if (threadIdx.x == 0) {
+        choose_grid(L.g, t, L.sch, L.fft_len);
+        L.g->counter2 = 0u;
+    }
+    __syncthreads();
+    if (L.g->tw_dirty) make_twiddles(L.tw, L.g->M);
 }
 
-// gather of the potentials + sparse attraction + gains/momentum step for T lanes per point; FP64 column sums of
-// the new layout for the recentring (the last block turns them into the mean and advances the iteration)
-template <int NI, int T>
-__global__ void __launch_bounds__(kThreads) loop_iter_kernel(const float2* __restrict__ Ycur, float2* __restrict__ Ynext,
-                                                             float2* __restrict__ U, float2* __restrict__ G,
-                                                             const int32_t* __restrict__ ip, const int32_t* __restrict__ ix,
-                                                             const float* __restrict__ P, int64_t n,
-                                                             GridDesc* __restrict__ gd, const float* __restrict__ phi,
-                                                             int pitchP, TsneSched s, double2* __restrict__ mpart) {
+// The spread of the charges (1, x, y) of a layout's points, recentred on the way (Ycur = Ynext - mean): one thread per
+// point, nodes accumulated with vector float atomics. Warps whose 32 points share one box (the dense case:
+// early-exaggeration layouts put everything in a few boxes) first reduce the node values with shuffles, so one atomic
+// per node replaces 32. Layout blockIdx.y.
+template <int NI, bool MANY>
+__global__ void __launch_bounds__(256) loop_spread_kernel(const __grid_constant__ LoopArgs args) {
+    const LoopDesc& L = MANY ? args.many[blockIdx.y] : args.one;
+    const GridDesc* gd = L.g;
+    const float xmin = gd->xmin, ymin = gd->ymin, width = gd->width, inv_w = gd->inv_width;
+    const int nb = gd->n_boxes;
+    const bool rc = gd->recentre != 0;
+    const float mx = gd->mean[0], my = gd->mean[1];
+    float4* const W = L.W;
+    const int pitch = L.Nmax;
+    const int lane = threadIdx.x & 31;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t base = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < L.n; base += stride) {
+        const int64_t i = base + lane;
+        const bool act = i < L.n;
+        float x = 0.f, y = 0.f;
+        if (act) {
+            const float2 p = L.Ynext[i];
+            x = p.x; y = p.y;
+            if (rc) { x = __fsub_rn(x, mx); y = __fsub_rn(y, my); }
+            L.Ycur[i] = make_float2(x, y);
+        }
+        int bx = 0, by = 0;
+        float wx[NI], wy[NI];
+        locate<NI>(x, y, xmin, ymin, width, inv_w, nb, bx, by, wx, wy);
+        const int key = act ? bx * nb + by : -1;
+        const int key0 = __shfl_sync(0xffffffffu, key, 0);
+        const bool one_box = __all_sync(0xffffffffu, act && key == key0) != 0;
+        if (one_box) {
+            // whole warp in one box: reduce per node, lane q issues node q
+#pragma unroll
+            for (int a = 0; a < NI; ++a) {
+#pragma unroll
+                for (int b = 0; b < NI; ++b) {
+                    const float w = wx[a] * wy[b];
+                    float s0 = w, s1 = w * x, s2 = w * y;
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) {
+                        s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+                        s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+                        s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+                    }
+                    if (lane == ((a * NI + b) & 31))
+                        atomicAdd(&W[(size_t)(bx * NI + a) * pitch + by * NI + b], make_float4(s0, s1, s2, 0.f));
+                }
+            }
+        } else if (act) {
+#pragma unroll
+            for (int a = 0; a < NI; ++a) {
+#pragma unroll
+                for (int b = 0; b < NI; ++b) {
+                    const float w = wx[a] * wy[b];
+                    atomicAdd(&W[(size_t)(bx * NI + a) * pitch + by * NI + b], make_float4(w, w * x, w * y, 0.f));
+                }
+            }
+        }
+    }
+}
+
+// gather of the potentials + sparse attraction + gains/momentum step for T lanes per point; FP64 column sums and the
+// bounding box of the new layout: the last block turns them into the mean (the pending recentring), the recentred box
+// (subtracting the mean rounds monotonically, so the box of the recentred points is the recentred box) and the next
+// iteration's grid, and advances the iteration. Layout first + blockIdx.y.
+// (MANY: several layouts. A single one's addresses are the launch's constants, which leaves 64 registers, four blocks per
+// SM; read from a descriptor they take 100.)
+template <int NI, int T, bool MANY>
+__global__ void __launch_bounds__(kThreads) loop_iter_kernel(const __grid_constant__ LoopArgs args, int first) {
     __shared__ double2 red[kThreads / 32];
     __shared__ int is_last;
+    const LoopDesc& L = MANY ? args.many[first + blockIdx.y] : args.one;
+    GridDesc* const gd = L.g;
+    const float2* __restrict__ Ycur = L.Ycur;
+    float2* __restrict__ Ynext = L.Ynext;
+    float2* __restrict__ U = L.U;
+    float2* __restrict__ G = L.G;
+    const int32_t* __restrict__ ip = L.ip;
+    const int32_t* __restrict__ ix = L.ix;
+    const float* __restrict__ P = L.P;
+    const float* __restrict__ phi = L.phi;
+    const int64_t n = L.n;
+    const int pitchP = L.Nmax;
+    const TsneSched s = L.sch;
     const int it = gd->iter;
     const bool early = it < s.early_iter;
     const float rho = early ? s.early_exag : s.exag;
@@ -250,6 +348,7 @@ __global__ void __launch_bounds__(kThreads) loop_iter_kernel(const float2* __res
     const size_t plane = (size_t)pitchP * pitchP;
     const int lg = threadIdx.x % T;
     const unsigned gmask = (T == 32) ? 0xffffffffu : (((1u << T) - 1u) << ((threadIdx.x & 31) / T * T));
+    BBox box{INFINITY, INFINITY, -INFINITY, -INFINITY};
     double sx = 0.0, sy = 0.0;
     const int64_t groups = (int64_t)gridDim.x * (blockDim.x / T);
     for (int64_t i = (int64_t)blockIdx.x * (blockDim.x / T) + threadIdx.x / T; i < n; i += groups) {
@@ -330,6 +429,7 @@ __global__ void __launch_bounds__(kThreads) loop_iter_kernel(const float2* __res
             Ynext[i] = make_float2(nx, ny);
             U[i] = u; G[i] = gn;
             sx += (double)nx; sy += (double)ny;
+            box = bbox_merge(box, BBox{nx, ny, nx, ny});
         }
     }
 #pragma unroll
@@ -338,11 +438,12 @@ __global__ void __launch_bounds__(kThreads) loop_iter_kernel(const float2* __res
         sy += __shfl_xor_sync(0xffffffffu, sy, o);
     }
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = make_double2(sx, sy);
-    __syncthreads();
+    box = block_bbox(box);
     if (threadIdx.x == 0) {
         double2 t = make_double2(0.0, 0.0);
         for (int w = 0; w < (int)(blockDim.x >> 5); ++w) { t.x += red[w].x; t.y += red[w].y; }
-        mpart[blockIdx.x] = t;
+        L.mean_part[blockIdx.x] = t;
+        L.box_part[blockIdx.x] = make_float4(box.x0, box.y0, box.x1, box.y1);
         __threadfence();
         is_last = atomicAdd(&gd->counter, 1u) == gridDim.x - 1;
     }
@@ -353,7 +454,7 @@ __global__ void __launch_bounds__(kThreads) loop_iter_kernel(const float2* __res
     // same bits from run to run)
     double tx = 0.0, ty = 0.0;
     for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
-        const double2 v = __ldcg(&mpart[b]);
+        const double2 v = __ldcg(&L.mean_part[b]);
         tx += v.x; ty += v.y;
     }
 #pragma unroll
@@ -363,15 +464,21 @@ __global__ void __launch_bounds__(kThreads) loop_iter_kernel(const float2* __res
     }
     __syncthreads();
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = make_double2(tx, ty);
+    BBox t = merge_boxes(L.box_part);
+    if (threadIdx.x == 0) {
+        tx = 0.0; ty = 0.0;
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) { tx += red[w].x; ty += red[w].y; }
+        const float mx = (float)(tx / (double)n), my = (float)(ty / (double)n);
+        gd->mean[0] = mx;
+        gd->mean[1] = my;
+        gd->recentre = 1;
+        t = BBox{__fsub_rn(t.x0, mx), __fsub_rn(t.y0, my), __fsub_rn(t.x1, mx), __fsub_rn(t.y1, my)};
+        choose_grid(gd, t, s, L.fft_len);
+        gd->iter = it + 1;
+        gd->counter = 0u;
+    }
     __syncthreads();
-    if (threadIdx.x != 0) return;
-    tx = 0.0; ty = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) { tx += red[w].x; ty += red[w].y; }
-    gd->mean[0] = (float)(tx / (double)n);
-    gd->mean[1] = (float)(ty / (double)n);
-    gd->recentre = 1;
-    gd->iter = it + 1;
-    gd->counter = 0u;
+    if (gd->tw_dirty) make_twiddles(L.tw, gd->M);
 }
 
 __global__ void finish_layout_kernel(const float2* __restrict__ Ynext, float2* __restrict__ Yout, int64_t n,
@@ -553,45 +660,60 @@ __global__ void finish_layout_perm_kernel(const float2* __restrict__ Ynext, cons
     }
 }
 
-template <int NI, int T>
-void launch_iter_t(TsneDev& d, cudaStream_t st) {
-    loop_iter_kernel<NI, T><<<d.blocks_iter, kThreads, 0, st>>>(
-        d.Ycur.as<float2>(), d.Ynext.as<float2>(), d.U.as<float2>(), d.G.as<float2>(), d.ip.as<int32_t>(),
-        d.ix.as<int32_t>(), d.P.as<float>(), d.n, d.g(), d.rb.phi.as<float>(), d.rb.Nmax, d.sch,
-        d.mean_part.as<double2>());
+// The iteration kernel over `count` layouts from `first` on: the grid is one resident wave (the kernel loops over rows),
+// so no second partial wave idles the device before the last-block reduction. With few layouts each gets blocks for
+// its rows; a batch shares the wave.
+constexpr int kIterBlocksMax = 8 * kNumSMs;   // partials a layout holds
+
+template <int NI, int T, bool MANY>
+int iter_resident() {
+    static thread_local int dev_known = -1, blocks = 0;
+    int dev = 0;
+    MGB_CUDA(cudaGetDevice(&dev));
+    if (dev != dev_known) {
+        int per_sm = 0;
+        MGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, loop_iter_kernel<NI, T, MANY>, kThreads, 0));
+        blocks = std::max(1, std::min(per_sm, kIterBlocksMax / kNumSMs)) * kNumSMs;
+        dev_known = dev;
+    }
+    return blocks;
 }
 
-// resident blocks of the iteration kernel for (NI, T): the grid is one resident wave (the kernel loops over
-// rows), so no second partial wave idles the device before the last-block reduction
 template <int NI, int T>
-int iter_blocks_t() {
-    int per_sm = 0;
-    MGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, loop_iter_kernel<NI, T>, kThreads, 0));
-    return std::max(1, per_sm) * kNumSMs;
+void launch_iter_t(const LoopArgs& a, int first, int count, int64_t n, cudaStream_t st) {
+    const int resident = a.many ? iter_resident<NI, T, true>() : iter_resident<NI, T, false>();
+    const int bx = std::max(1, std::min(grid_blocks(n, kThreads / T, 8), ceil_div(resident, count)));
+    if (a.many) loop_iter_kernel<NI, T, true><<<dim3(bx, count), kThreads, 0, st>>>(a, first);
+    else loop_iter_kernel<NI, T, false><<<dim3(bx, count), kThreads, 0, st>>>(a, first);
 }
 template <int NI>
-int iter_blocks_ni(int tpr) {
+void launch_iter_ni(const LoopArgs& a, int first, int count, int tpr, int64_t n, cudaStream_t st) {
     switch (tpr) {
-        case 1: return iter_blocks_t<NI, 1>();
-        case 2: return iter_blocks_t<NI, 2>();
-        case 4: return iter_blocks_t<NI, 4>();
-        case 8: return iter_blocks_t<NI, 8>();
-        case 16: return iter_blocks_t<NI, 16>();
-        default: return iter_blocks_t<NI, 32>();
+        case 1: launch_iter_t<NI, 1>(a, first, count, n, st); break;
+        case 2: launch_iter_t<NI, 2>(a, first, count, n, st); break;
+        case 4: launch_iter_t<NI, 4>(a, first, count, n, st); break;
+        case 8: launch_iter_t<NI, 8>(a, first, count, n, st); break;
+        case 16: launch_iter_t<NI, 16>(a, first, count, n, st); break;
+        default: launch_iter_t<NI, 32>(a, first, count, n, st); break;
     }
 }
-
 template <int NI>
-void launch_iter_ni(TsneDev& d, cudaStream_t st) {
-    switch (d.tpr) {
-        case 1: launch_iter_t<NI, 1>(d, st); break;
-        case 2: launch_iter_t<NI, 2>(d, st); break;
-        case 4: launch_iter_t<NI, 4>(d, st); break;
-        case 8: launch_iter_t<NI, 8>(d, st); break;
-        case 16: launch_iter_t<NI, 16>(d, st); break;
-        default: launch_iter_t<NI, 32>(d, st); break;
-    }
+void launch_spread_ni(const LoopArgs& a, int64_t n, cudaStream_t st) {
+    const int bx = std::max(1, std::min(grid_blocks(n, 256, 16), ceil_div(16 * kNumSMs, a.count)));
+    if (a.many) loop_spread_kernel<NI, true><<<dim3(bx, a.count), 256, 0, st>>>(a);
+    else loop_spread_kernel<NI, false><<<dim3(bx, 1), 256, 0, st>>>(a);
 }
+#define MGB_LOOP_NI(ni, F, ...)                     \
+    switch (ni) {                                   \
+        case 1: F<1>(__VA_ARGS__); break;           \
+        case 2: F<2>(__VA_ARGS__); break;           \
+        case 3: F<3>(__VA_ARGS__); break;           \
+        case 4: F<4>(__VA_ARGS__); break;           \
+        case 5: F<5>(__VA_ARGS__); break;           \
+        case 6: F<6>(__VA_ARGS__); break;           \
+        case 7: F<7>(__VA_ARGS__); break;           \
+        default: F<8>(__VA_ARGS__); break;          \
+    }
 
 }  // namespace
 
@@ -703,21 +825,8 @@ void TsneDev::init(const int32_t* ip_h, const int32_t* ix_h, const float* P_h, i
     rep_prepare_device_spectra(rb);
     gdesc.ensure(sizeof(GridDesc));
     MGB_CUDA(cudaMemsetAsync(gdesc.p, 0, sizeof(GridDesc), st));
-    blocks_bbox = grid_blocks(n, kThreads, 4);
-    int resident = 0;
-    switch (s.ni) {
-        case 1: resident = iter_blocks_ni<1>(tpr); break;
-        case 2: resident = iter_blocks_ni<2>(tpr); break;
-        case 3: resident = iter_blocks_ni<3>(tpr); break;
-        case 4: resident = iter_blocks_ni<4>(tpr); break;
-        case 5: resident = iter_blocks_ni<5>(tpr); break;
-        case 6: resident = iter_blocks_ni<6>(tpr); break;
-        case 7: resident = iter_blocks_ni<7>(tpr); break;
-        default: resident = iter_blocks_ni<8>(tpr); break;
-    }
-    blocks_iter = std::min(grid_blocks(n, kThreads / tpr, 8), resident);
-    bbox_part.ensure(sizeof(BBox) * blocks_bbox);
-    mean_part.ensure(sizeof(double2) * blocks_iter);
+    box_part.ensure(sizeof(float4) * kIterBlocksMax);
+    mean_part.ensure(sizeof(double2) * kIterBlocksMax);
     if (graph && signature() != graph_sig) { cudaGraphExecDestroy(graph); graph = nullptr; }
 }
 
@@ -776,33 +885,57 @@ void TsneDev::get_layout(float* Y, bool host, cudaStream_t st) {
     }
 }
 
-void TsneDev::iterate(cudaStream_t st, cudaEvent_t* ev) {
+LoopDesc TsneDev::desc() {
+    LoopDesc d = rep_desc(rb, g(), n);
+    d.Ycur = Ycur.as<float2>(); d.Ynext = Ynext.as<float2>(); d.U = U.as<float2>(); d.G = G.as<float2>();
+    d.ip = ip.as<int32_t>(); d.ix = ix.as<int32_t>(); d.P = P.as<float>();
+    d.box_part = box_part.as<float4>(); d.mean_part = mean_part.as<double2>();
+    d.sch = sch; d.dof = (double)dof;
+    return d;
+}
+
+void loop_start(const LoopArgs& a, const LoopSizes& z, cudaStream_t st) {
+    const int bx = std::max(1, std::min(grid_blocks(z.n, kThreads, 4), ceil_div(4 * kNumSMs, a.count)));
+    loop_start_kernel<<<dim3(bx, a.count), kThreads, 0, st>>>(a);
+    MGB_LAUNCH_CHECK();
+}
+
+void loop_iterate(const LoopArgs& a, const LoopSizes& z, const LaneRun* runs, int n_runs, cudaStream_t st,
+                  cudaStream_t side, cudaEvent_t fork, cudaEvent_t join, cudaEvent_t* ev) {
     auto mark = [&](int k) { if (ev) MGB_CUDA(cudaEventRecord(ev[k], st)); };
     mark(0);
-    loop_bbox_kernel<<<blocks_bbox, kThreads, 0, st>>>(Ynext.as<float2>(), Ycur.as<float2>(), n, g(),
-                                                      bbox_part.as<BBox>(), sch, rb.fft_len_table.as<int>());
+    // beside the spread, where their blocks pass between its many small ones: beside the forward rows, whose blocks fill
+    // the device for the whole pass, they waited for those to end and held the columns up (1,000,000 points: 30 us)
+    if (side) {
+        MGB_CUDA(cudaEventRecord(fork, st));
+        MGB_CUDA(cudaStreamWaitEvent(side, fork, 0));
+        rep_update_spectra(a, z.Mmax, side);
+        MGB_CUDA(cudaEventRecord(join, side));
+    }
+    MGB_LOOP_NI(z.ni, launch_spread_ni, a, z.n, st);
     MGB_LAUNCH_CHECK();
     mark(1);
-    rep_twiddles(g(), rb, st, false);
+    if (!side) rep_update_spectra(a, z.Mmax, st);
     mark(2);
-    rep_update_spectra(g(), rb, dof, st);
+    rep_row_fwd3(a, z, st);
     mark(3);
-    rep_spread(Ycur.as<float2>(), n, g(), rb, st);
+    if (side) MGB_CUDA(cudaStreamWaitEvent(st, join, 0));
+    rep_col3(a, z, st);
     mark(4);
-    rep_convolve(g(), rb, n, st, ev ? ev + 5 : nullptr);
-    switch (ni) {
-        case 1: launch_iter_ni<1>(*this, st); break;
-        case 2: launch_iter_ni<2>(*this, st); break;
-        case 3: launch_iter_ni<3>(*this, st); break;
-        case 4: launch_iter_ni<4>(*this, st); break;
-        case 5: launch_iter_ni<5>(*this, st); break;
-        case 6: launch_iter_ni<6>(*this, st); break;
-        case 7: launch_iter_ni<7>(*this, st); break;
-        default: launch_iter_ni<8>(*this, st); break;
+    rep_row_inv3(a, z, st);
+    mark(5);
+    for (int q = 0; q < n_runs; ++q) {
+        MGB_LOOP_NI(z.ni, launch_iter_ni, a, runs[q].first, runs[q].count, runs[q].tpr, z.n, st);
+        MGB_LAUNCH_CHECK();
     }
-    MGB_LAUNCH_CHECK();
-    mark(8);
+    mark(6);
 }
+
+namespace {
+// what a single layout's launches take
+LoopArgs one_layout(TsneDev& d) { return LoopArgs{d.desc(), nullptr, 1}; }
+LoopSizes sizes_of(const TsneDev& d) { return LoopSizes{d.n, d.rb.Nmax, d.rb.Mmax, d.rb.Mp3max, d.ni}; }
+}  // namespace
 
 bool TsneDev::reorder_due(int i) const {
     return reorder_every > 0 && n >= kReorderMinPoints && n <= INT32_MAX && i % reorder_every == 1;
@@ -852,38 +985,24 @@ void TsneDev::reorder(cudaStream_t st) {
 
 void TsneDev::run(int n_iter, bool use_graph, cudaStream_t st) {
     if (n_iter <= 0) return;
+    const LoopArgs a = one_layout(*this);
+    const LoopSizes z = sizes_of(*this);
+    const LaneRun lanes{0, 1, tpr};
+    loop_start(a, z, st);
     if (!use_graph) {
         for (int i = 0; i < n_iter; ++i) {
             if (reorder_due(i)) reorder(st);
-            iterate(st);
+            loop_iterate(a, z, &lanes, 1, st, nullptr, nullptr, nullptr, nullptr);
         }
         return;
     }
     if (graph && graph_stream != st) { cudaGraphExecDestroy(graph); graph = nullptr; }
     if (!graph) {
-        // capture on a private stream (capture on the legacy default stream is not allowed), replay on st
-        cudaStream_t cap;
-        MGB_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
-        cudaGraph_t gr = nullptr;
-        try {
-            MGB_CUDA(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
-            const uint64_t before = launch_count();
-            iterate(cap);
-            graph_kernels = launch_count() - before;
-            MGB_CUDA(cudaStreamEndCapture(cap, &gr));
-        } catch (...) {
-            cudaGraph_t tmp = nullptr;
-            cudaStreamEndCapture(cap, &tmp);
-            if (tmp) cudaGraphDestroy(tmp);
-            cudaStreamDestroy(cap);
-            throw;
-        }
-        cudaStreamDestroy(cap);
-        MGB_CUDA(cudaGraphInstantiate(&graph, gr, 0));
-        cudaGraphDestroy(gr);
+        graph = capture_loop([&](cudaStream_t cap, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join) {
+            loop_iterate(a, z, &lanes, 1, cap, side, fork, join, nullptr);
+        }, graph_kernels);
         graph_stream = st;
         graph_sig = signature();
-        count_launch(0 - graph_kernels);   // captured, not run: the replays below count them
     }
     for (int i = 0; i < n_iter; ++i) {
         if (reorder_due(i)) reorder(st);
@@ -892,31 +1011,79 @@ void TsneDev::run(int n_iter, bool use_graph, cudaStream_t st) {
     }
 }
 
+// one iteration captured on private streams (capture on the legacy default stream is not allowed); kernels = the
+// launches it holds (captured, not run: the replays count them)
+cudaGraphExec_t capture_loop(const std::function<void(cudaStream_t, cudaStream_t, cudaEvent_t, cudaEvent_t)>& body,
+                             uint64_t& kernels) {
+    struct Owned {
+        cudaStream_t cap = nullptr, side = nullptr;
+        cudaEvent_t fork = nullptr, join = nullptr;
+        cudaGraph_t gr = nullptr;
+        ~Owned() {
+            if (gr) cudaGraphDestroy(gr);
+            if (fork) cudaEventDestroy(fork);
+            if (join) cudaEventDestroy(join);
+            if (side) cudaStreamDestroy(side);
+            if (cap) cudaStreamDestroy(cap);
+        }
+    } o;
+    MGB_CUDA(cudaStreamCreateWithFlags(&o.cap, cudaStreamNonBlocking));
+    MGB_CUDA(cudaStreamCreateWithFlags(&o.side, cudaStreamNonBlocking));
+    MGB_CUDA(cudaEventCreateWithFlags(&o.fork, cudaEventDisableTiming));
+    MGB_CUDA(cudaEventCreateWithFlags(&o.join, cudaEventDisableTiming));
+    MGB_CUDA(cudaStreamBeginCapture(o.cap, cudaStreamCaptureModeThreadLocal));
+    const uint64_t before = launch_count();
+    try {
+        body(o.cap, o.side, o.fork, o.join);
+    } catch (...) {
+        cudaStreamEndCapture(o.cap, &o.gr);
+        cudaGetLastError();
+        throw;
+    }
+    kernels = launch_count() - before;
+    count_launch(0 - kernels);
+    MGB_CUDA(cudaStreamEndCapture(o.cap, &o.gr));
+    cudaGraphExec_t exec = nullptr;
+    MGB_CUDA(cudaGraphInstantiate(&exec, o.gr, 0));
+    return exec;
+}
+
 void TsneDev::run_profiled(int n_iter, cudaStream_t st, double* stage_ms, int* grid) {
+    const LoopArgs a = one_layout(*this);
+    const LoopSizes z = sizes_of(*this);
+    const LaneRun lanes{0, 1, tpr};
+    // the reported stages: 0 bbox + grid choice (the first grid; the later ones are the last stage's), 1 twiddles (the
+    // spread's), 2 kernel spectra, 3 spread, 4 forward rows, 5 columns, 6 inverse rows, 7 gather + step, 8 all
+    static const int slot[6] = {3, 2, 4, 5, 6, 7};
     cudaEvent_t ev[9];
     for (auto& e : ev) MGB_CUDA(cudaEventCreate(&e));
+    auto between = [&](int x, int y) {
+        float ms = 0.f;
+        MGB_CUDA(cudaEventElapsedTime(&ms, ev[x], ev[y]));
+        return (double)ms;
+    };
     try {
+        if (n_iter > 0) {
+            MGB_CUDA(cudaEventRecord(ev[0], st));
+            loop_start(a, z, st);
+            MGB_CUDA(cudaEventRecord(ev[1], st));
+            MGB_CUDA(cudaEventSynchronize(ev[1]));
+            stage_ms[0] += between(0, 1);
+            stage_ms[8] += between(0, 1);
+        }
         for (int it = 0; it < n_iter; ++it) {
-            float ro = 0.f;
-            if (reorder_due(it)) {   // counted with stage 0 (bbox + grid choice) and in the total
-                MGB_CUDA(cudaEventRecord(ev[0], st));
+            if (reorder_due(it)) {   // counted with stage 0 and in the total
+                MGB_CUDA(cudaEventRecord(ev[7], st));
                 reorder(st);
-                MGB_CUDA(cudaEventRecord(ev[1], st));
-                MGB_CUDA(cudaEventSynchronize(ev[1]));
-                MGB_CUDA(cudaEventElapsedTime(&ro, ev[0], ev[1]));
-                stage_ms[0] += ro;
-                stage_ms[8] += ro;
+                MGB_CUDA(cudaEventRecord(ev[8], st));
+                MGB_CUDA(cudaEventSynchronize(ev[8]));
+                stage_ms[0] += between(7, 8);
+                stage_ms[8] += between(7, 8);
             }
-            iterate(st, ev);
-            MGB_CUDA(cudaEventSynchronize(ev[8]));
-            for (int k = 0; k < 8; ++k) {
-                float ms = 0.f;
-                MGB_CUDA(cudaEventElapsedTime(&ms, ev[k], ev[k + 1]));
-                stage_ms[k] += ms;
-            }
-            float all = 0.f;
-            MGB_CUDA(cudaEventElapsedTime(&all, ev[0], ev[8]));
-            stage_ms[8] += all;
+            loop_iterate(a, z, &lanes, 1, st, nullptr, nullptr, nullptr, ev);
+            MGB_CUDA(cudaEventSynchronize(ev[6]));
+            for (int k = 0; k < 6; ++k) stage_ms[slot[k]] += between(k, k + 1);
+            stage_ms[8] += between(0, 6);
         }
         GridDesc gh;
         MGB_CUDA(cudaMemcpy(&gh, gdesc.p, sizeof(GridDesc), cudaMemcpyDeviceToHost));

@@ -2,6 +2,7 @@
 // the whole optimisation loop of magnet/tsne.py:132-214 (common path) kept on the device.
 #pragma once
 #include "fftrep.cuh"
+#include <functional>
 #include <string>
 
 namespace mgb {
@@ -18,13 +19,6 @@ void mid_spring_dev(const float* Y, const int32_t* pairs, float* grad, int64_t n
                     cudaStream_t s);
 void center_scale_dev(float* Y, int64_t n, int dim, double target_std, DevBuf& scratch, cudaStream_t s);
 
-struct TsneSched {
-    int early_iter;
-    float early_exag, exag, mom0, mom1, lr, inv_dof;
-    double box_width;
-    int min_boxes, max_boxes, ni;
-};
-
 // Device-resident state of one t-SNE layout: the layout double buffer, the optimiser state, the normalised
 // affinities and the repulsion buffers. One instance per stream.
 struct TsneDev {
@@ -32,13 +26,12 @@ struct TsneDev {
     int ni = 3, tpr = 8;
     float dof = 1.f;
     TsneSched sch{};
-    DevBuf Ycur, Ynext, U, G, ip, ix, P, gdesc, bbox_part, mean_part;
+    DevBuf Ycur, Ynext, U, G, ip, ix, P, gdesc, box_part, mean_part;
     RepBuffers rb;
     cudaGraphExec_t graph = nullptr;
     cudaStream_t graph_stream = nullptr;
     uint64_t graph_kernels = 0;         // kernel nodes of the captured iteration
     std::string graph_sig;              // sizes, schedule and buffer addresses the graph was captured with
-    int blocks_iter = 0, blocks_bbox = 0;
     // spatial order of the points (the loop of a large layout): row r of every per-point array holds the caller's
     // point perm[r]; the affinity rows and their column indices are relabelled to match. Set by reorder(),
     // undone by set_layout / get_layout, so callers always see their own order.
@@ -51,8 +44,7 @@ struct TsneDev {
               const TsneSched& s, float dof, int threads_per_row, cudaStream_t st);
     void set_layout(const float* Y, bool host_ptr, cudaStream_t st);   // also resets update = 0, gains = 1
     void get_layout(float* Y, bool host_ptr, cudaStream_t st);         // applies the pending recentring
-    // one iteration, plain launches; with ev (8 events) the stage boundaries are recorded
-    void iterate(cudaStream_t st, cudaEvent_t* ev = nullptr);
+    LoopDesc desc();   // what the loop's kernels read
     void run(int n_iter, bool use_graph, cudaStream_t st);
     // plain launches with per-stage event timing; stage_ms[0..7] += stage times, grid[4] = last grid
     void run_profiled(int n_iter, cudaStream_t st, double* stage_ms, int* grid);
@@ -63,5 +55,21 @@ struct TsneDev {
     std::string signature() const;
     GridDesc* g() { return gdesc.as<GridDesc>(); }
 };
+
+// The loop's launches over the layouts of `a` (all of one n_interp).
+// the first grid of every layout, from its starting positions; the later ones come out of the iterations
+void loop_start(const LoopArgs& a, const LoopSizes& z, cudaStream_t st);
+// one iteration; layouts [from[q], from[q + 1]) take tprs[q] lanes per row (runs of equal lanes). `side` (or null)
+// takes the kernel spectra off the iteration's path (a stream of the same capture); with ev (8 events) the stage
+// boundaries are recorded: grid, spread, spectra, forward rows, columns, inverse rows, gather + step.
+struct LaneRun {
+    int first, count, tpr;
+};
+void loop_iterate(const LoopArgs& a, const LoopSizes& z, const LaneRun* runs, int n_runs, cudaStream_t st,
+                  cudaStream_t side, cudaEvent_t fork, cudaEvent_t join, cudaEvent_t* ev);
+
+// a captured iteration: body(stream, side stream, fork, join) launches it
+cudaGraphExec_t capture_loop(const std::function<void(cudaStream_t, cudaStream_t, cudaEvent_t, cudaEvent_t)>& body,
+                             uint64_t& kernels);
 
 }  // namespace mgb

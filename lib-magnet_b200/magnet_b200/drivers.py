@@ -182,7 +182,7 @@ def optimize_tsne_batch(Ps, Ys, n_iter=500, early_iter=None, early_exaggeration=
                         learning_rate=None, momentum=(0.5, 0.8), n_interp=3, box_width=0.7, dof=1.0,
                         max_boxes=None, threads_per_row=None, branches=None, autotune=True):
     """Many independent t-SNE passes (each the device loop of optimize_tsne, magnet/tsne.py:132-214) run together:
-    one CUDA graph holds one iteration of every layout as independent branches, replayed n_iter times. Ps: the
+    one CUDA graph holds one iteration of every layout, whose launches cover many layouts each, replayed n_iter times. Ps: the
     layouts' symmetric CSR affinities (each normalised to sum 1 inside), Ys: their (n_i, 2) float32 initial layouts
     (numpy or device arrays), updated in place and returned. early_iter None: min(250, n_iter // 3), MAGNET's
     default for loss="tsne" (magnet/__init__.py:640). The learning rate, when None, is each layout's own
