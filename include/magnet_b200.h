@@ -141,7 +141,7 @@ int mg_tsne_batch_create(int count, const int64_t* n, const int64_t* nnz, const 
                          const int32_t* const* indices, const float* const* P, const mg_tsne_params* p,
                          const int* max_boxes, int branches, mg_tsne_batch** out);
 /* Runs p->n_iter iterations of every layout from Y[i] ((n[i], 2), host or device), updated in place. Synchronous.
- * The first run on a stream captures the iteration graph. */
+ * The first run captures the iteration graph. */
 int mg_tsne_batch_run(mg_tsne_batch* b, float* const* Y);
 /* Layout count and kernels per replayed iteration (0 before the first run). */
 int mg_tsne_batch_size(const mg_tsne_batch* b, int* count, uint64_t* kernels_per_iteration);

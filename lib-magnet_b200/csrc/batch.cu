@@ -50,7 +50,6 @@ struct TsneBatch {
     std::vector<std::unique_ptr<Set>> sets;
     cudaEvent_t begin = nullptr;
     cudaGraphExec_t graph = nullptr;
-    cudaStream_t graph_stream = nullptr;
     uint64_t graph_kernels = 0;
     int n_iter = 0;
 
@@ -95,10 +94,9 @@ struct TsneBatch {
     }
 
     // one iteration of every layout as one graph: the sets are its branches
-    void capture(cudaStream_t st) {
-        if (graph && graph_stream == st) return;
-        if (graph) { cudaGraphExecDestroy(graph); graph = nullptr; }
-        graph = capture_loop([&](cudaStream_t cap, cudaStream_t, cudaEvent_t, cudaEvent_t) {
+    void capture() {
+        if (graph) return;   // (the executable may be launched on any stream)
+        capture_loop([&](cudaStream_t cap, cudaStream_t, cudaEvent_t, cudaEvent_t) {
             MGB_CUDA(cudaEventRecord(begin, cap));
             for (auto& s : sets) {
                 MGB_CUDA(cudaStreamWaitEvent(s->stream, begin, 0));
@@ -107,8 +105,7 @@ struct TsneBatch {
                 MGB_CUDA(cudaEventRecord(s->done, s->stream));
                 MGB_CUDA(cudaStreamWaitEvent(cap, s->done, 0));
             }
-        }, graph_kernels);
-        graph_stream = st;
+        }, graph, graph_kernels);
     }
 };
 
@@ -158,7 +155,7 @@ extern "C" int mg_tsne_batch_run(mg_tsne_batch* h, float* const* Y) {
             b.layouts[i]->set_layout(Y[i], !is_device_ptr(Y[i]), s);
         }
         if (b.n_iter > 0) {
-            b.capture(s);
+            b.capture();
             for (auto& q : b.sets) loop_start(q->args, q->sizes, s);
             for (int it = 0; it < b.n_iter; ++it) {
                 MGB_CUDA(cudaGraphLaunch(b.graph, s));

@@ -88,38 +88,64 @@ __device__ __forceinline__ float step_coord(float y, float& u, float& gain, floa
     return __fadd_rn(y, un);
 }
 
-// mode 0: grad = rho * A - F * inv_sumQ (tsne_step); mode 1: grad given (tsne_update)
-__global__ void step_kernel(float* __restrict__ Y, float* __restrict__ U, float* __restrict__ G,
-                            const float* __restrict__ A, const float* __restrict__ F, int64_t total, float rho,
-                            float inv_sumQ, float lr, float momentum, int mode) {
-    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < total; k += (int64_t)gridDim.x * blockDim.x) {
-        const float g_ = mode == 0 ? __fsub_rn(__fmul_rn(rho, A[k]), __fmul_rn(F[k], inv_sumQ)) : A[k];
-        float u = U[k], gain = G[k];
-        Y[k] = step_coord(Y[k], u, gain, g_, lr, momentum);
-        U[k] = u; G[k] = gain;
-    }
-}
-
-// column sums in FP64, one block per dimension, fixed order; then the mean as (float)(sum / n)
-__global__ void colmean_kernel(const float* __restrict__ Y, int64_t n, int dim, float* __restrict__ mean) {
-    __shared__ double red[kThreads / 32];
-    const int d = blockIdx.x;
-    double s = 0.0;
-    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) s += (double)Y[i * dim + d];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+// red[r * dim + c], r < rows, summed over r into red[c] in a fixed order; by the whole block
+__device__ __forceinline__ void column_sums(double* red, int rows, int dim) {
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
-        mean[d] = (float)(t / (double)n);
+    while (rows > 1) {
+        const int half = (rows + 1) / 2;
+        if ((int)threadIdx.x < (rows - half) * dim) red[threadIdx.x] += red[threadIdx.x + half * dim];
+        __syncthreads();
+        rows = half;
     }
 }
 
-__global__ void subtract_mean_kernel(float* __restrict__ Y, int64_t total, int dim, const float* __restrict__ mean) {
-    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < total; k += (int64_t)gridDim.x * blockDim.x)
-        Y[k] -= mean[k % dim];
+// mode 0: grad = rho * A - F * inv_sumQ (tsne_step); mode 1: grad given (tsne_update)
+// The FP64 column sums of the new positions are taken on the way: a thread stays in one column (the blocks advance by
+// whole rows), the last block turns the partial sums into the means (float)(sum / n). Bound by the 32 bytes per
+// coordinate it moves; with the means in a launch of one block per column, that launch alone took 132 us at 400,000
+// points (now 6 us in all, with the step).
+__global__ void __launch_bounds__(kThreads) step_kernel(float* __restrict__ Y, float* __restrict__ U, float* __restrict__ G,
+                                                        const float* __restrict__ A, const float* __restrict__ F,
+                                                        int64_t total, float rho, float inv_sumQ, float lr,
+                                                        float momentum, int mode, int dim, double* __restrict__ part,
+                                                        unsigned* __restrict__ counter, float* __restrict__ mean) {
+    __shared__ double red[kThreads];
+    __shared__ int is_last;
+    const int live = kThreads / dim * dim;
+    double sum = 0.0;
+    if ((int)threadIdx.x < live) {
+        for (int64_t k = (int64_t)blockIdx.x * live + threadIdx.x; k < total; k += (int64_t)gridDim.x * live) {
+            const float g_ = mode == 0 ? __fsub_rn(__fmul_rn(rho, A[k]), __fmul_rn(F[k], inv_sumQ)) : A[k];
+            float u = U[k], gain = G[k];
+            const float y = step_coord(Y[k], u, gain, g_, lr, momentum);
+            Y[k] = y; U[k] = u; G[k] = gain;
+            sum += (double)y;
+        }
+        red[threadIdx.x] = sum;
+    }
+    column_sums(red, live / dim, dim);
+    if ((int)threadIdx.x < dim) part[(int64_t)blockIdx.x * dim + threadIdx.x] = red[threadIdx.x];
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) is_last = atomicAdd(counter, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!is_last) return;
+    __threadfence();
+    sum = 0.0;
+    if ((int)threadIdx.x < live) {
+        for (int k = threadIdx.x; k < (int)gridDim.x * dim; k += live) sum += __ldcg(&part[k]);
+        red[threadIdx.x] = sum;
+    }
+    column_sums(red, live / dim, dim);
+    if ((int)threadIdx.x < dim) mean[threadIdx.x] = (float)(red[threadIdx.x] / (double)(total / dim));
+}
+
+__global__ void __launch_bounds__(kThreads) subtract_mean_kernel(float* __restrict__ Y, int64_t total, int dim,
+                                                                 const float* __restrict__ mean) {
+    const int live = kThreads / dim * dim;
+    if ((int)threadIdx.x >= live) return;
+    const float m = mean[threadIdx.x % dim];
+    for (int64_t k = (int64_t)blockIdx.x * live + threadIdx.x; k < total; k += (int64_t)gridDim.x * live) Y[k] -= m;
 }
 
 // ---------------------------------------------------------------------------------------------- bbox
@@ -556,7 +582,13 @@ __global__ void center_apply_kernel(float* __restrict__ Y, int64_t total, int di
         Y[k] = (Y[k] - st[k % dim]) * f;
 }
 
-__global__ void init_opt_state_kernel(float2* U, float2* G, int64_t n) {
+// update 0, gains 1; no pending recentring, iteration 0, empty spectrum and twiddle keys
+__global__ void init_opt_state_kernel(float2* U, float2* G, int64_t n, GridDesc* g) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        GridDesc zero{};
+        zero.key_nb = -1; zero.tw_M = -1;
+        *g = zero;
+    }
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         U[i] = make_float2(0.f, 0.f);
         G[i] = make_float2(1.f, 1.f);
@@ -735,13 +767,18 @@ static void step_common(float* Y, float* U, float* G, const float* A, const floa
                         float inv_sumQ, float lr, float momentum, int mode, DevBuf& scratch, cudaStream_t s) {
     const int64_t total = n * dim;
     if (total == 0) return;
-    step_kernel<<<grid_blocks(total, kThreads), kThreads, 0, s>>>(Y, U, G, A, F, total, rho, inv_sumQ, lr, momentum,
-                                                                  mode);
+    const int live = kThreads / dim * dim;
+    const int blocks = grid_blocks(total, live, 8);
+    // scratch: the means, the counter, the blocks' partial sums
+    char* base = static_cast<char*>(scratch.ensure(512 + sizeof(double) * dim * blocks));
+    float* mean = reinterpret_cast<float*>(base);
+    unsigned* counter = reinterpret_cast<unsigned*>(base + 256);
+    double* part = reinterpret_cast<double*>(base + 512);
+    MGB_CUDA(cudaMemsetAsync(counter, 0, sizeof(unsigned), s));
+    step_kernel<<<blocks, kThreads, 0, s>>>(Y, U, G, A, F, total, rho, inv_sumQ, lr, momentum, mode, dim, part, counter,
+                                            mean);
     MGB_LAUNCH_CHECK();
-    float* mean = static_cast<float*>(scratch.ensure(sizeof(float) * kMaxDim));
-    colmean_kernel<<<dim, kThreads, 0, s>>>(Y, n, dim, mean);
-    MGB_LAUNCH_CHECK();
-    subtract_mean_kernel<<<grid_blocks(total, kThreads), kThreads, 0, s>>>(Y, total, dim, mean);
+    subtract_mean_kernel<<<blocks, kThreads, 0, s>>>(Y, total, dim, mean);
     MGB_LAUNCH_CHECK();
 }
 
@@ -792,8 +829,8 @@ TsneDev::~TsneDev() {
     if (graph) cudaGraphExecDestroy(graph);
 }
 
-void TsneDev::init(const int32_t* ip_h, const int32_t* ix_h, const float* P_h, int64_t n_, int64_t nnz_, bool host,
-                   const TsneSched& s, float dof_, int threads_per_row, cudaStream_t st) {
+void TsneDev::init(const int32_t* ip_d, const int32_t* ix_d, int64_t n_, int64_t nnz_, const TsneSched& s,
+                   float dof_, int threads_per_row, cudaStream_t st) {
     require(n_ >= 1, "the layout needs at least one point");
     require(s.ni >= 1 && s.ni <= 8, "n_interp must be between 1 and 8");
     require(s.min_boxes >= 1 && s.max_boxes >= s.min_boxes, "invalid box limits");
@@ -810,30 +847,25 @@ void TsneDev::init(const int32_t* ip_h, const int32_t* ix_h, const float* P_h, i
         tpr = threads_per_row >= 32 ? 32 : threads_per_row >= 16 ? 16 : threads_per_row >= 8 ? 8
             : threads_per_row >= 4 ? 4 : threads_per_row >= 2 ? 2 : 1;
     }
-    const cudaMemcpyKind kind = host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
     Ycur.ensure(sizeof(float2) * n); Ynext.ensure(sizeof(float2) * n);
     U.ensure(sizeof(float2) * n); G.ensure(sizeof(float2) * n);
     ip.ensure(sizeof(int32_t) * (n + 1)); ix.ensure(sizeof(int32_t) * std::max<int64_t>(nnz, 1));
     P.ensure(sizeof(float) * std::max<int64_t>(nnz, 1));
-    MGB_CUDA(cudaMemcpyAsync(ip.p, ip_h, sizeof(int32_t) * (n + 1), kind, st));
-    if (nnz > 0) {
-        MGB_CUDA(cudaMemcpyAsync(ix.p, ix_h, sizeof(int32_t) * nnz, kind, st));
-        MGB_CUDA(cudaMemcpyAsync(P.p, P_h, sizeof(float) * nnz, kind, st));
-    }
+    MGB_CUDA(cudaMemcpyAsync(ip.p, ip_d, sizeof(int32_t) * (n + 1), cudaMemcpyDeviceToDevice, st));
+    if (nnz > 0) MGB_CUDA(cudaMemcpyAsync(ix.p, ix_d, sizeof(int32_t) * nnz, cudaMemcpyDeviceToDevice, st));
     const int Nmax = s.max_boxes * s.ni;
     rb.alloc(Nmax, next_fft_len(2 * Nmax), s.ni);
     rep_prepare_device_spectra(rb);
     gdesc.ensure(sizeof(GridDesc));
-    MGB_CUDA(cudaMemsetAsync(gdesc.p, 0, sizeof(GridDesc), st));
     box_part.ensure(sizeof(float4) * kIterBlocksMax);
     mean_part.ensure(sizeof(double2) * kIterBlocksMax);
-    if (graph && signature() != graph_sig) { cudaGraphExecDestroy(graph); graph = nullptr; }
+    graph_stale = graph && signature() != graph_sig;
 }
 
 std::string TsneDev::signature() const {
     char buf[512];
-    std::snprintf(buf, sizeof(buf), "%lld %lld %d %d %g %d %g %g %g %g %g %g %.17g %d %d %d %p %p %p %p %p %p %p %p %p %p %d %d",
-                  (long long)n, (long long)nnz, ni, tpr, (double)dof, sch.early_iter, (double)sch.early_exag,
+    std::snprintf(buf, sizeof(buf), "%lld %d %d %g %d %g %g %g %g %g %g %.17g %d %d %d %p %p %p %p %p %p %p %p %p %p %d %d",
+                  (long long)n, ni, tpr, (double)dof, sch.early_iter, (double)sch.early_exag,
                   (double)sch.exag, (double)sch.mom0, (double)sch.mom1, (double)sch.lr, (double)sch.inv_dof,
                   sch.box_width, sch.min_boxes, sch.max_boxes, sch.ni, Ycur.p, Ynext.p, U.p, G.p, ip.p, ix.p, P.p,
                   gdesc.p, rb.W.p, rb.phi.p, rb.Nmax, rb.Mmax);
@@ -853,13 +885,8 @@ void TsneDev::set_layout(const float* Y, bool host, cudaStream_t st) {
         MGB_CUDA(cudaMemcpyAsync(Ynext.p, Y, sizeof(float2) * n, host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice,
                                  st));
     }
-    init_opt_state_kernel<<<grid_blocks(n, kThreads), kThreads, 0, st>>>(U.as<float2>(), G.as<float2>(), n);
+    init_opt_state_kernel<<<grid_blocks(n, kThreads), kThreads, 0, st>>>(U.as<float2>(), G.as<float2>(), n, g());
     MGB_LAUNCH_CHECK();
-    // no pending recentring, iteration 0, empty spectrum and twiddle keys
-    GridDesc zero{};
-    zero.key_nb = -1; zero.tw_M = -1;
-    MGB_CUDA(cudaMemcpyAsync(gdesc.p, &zero, sizeof(GridDesc), cudaMemcpyHostToDevice, st));
-    MGB_CUDA(cudaStreamSynchronize(st));   // `zero` lives on this stack frame
 }
 
 void TsneDev::get_layout(float* Y, bool host, cudaStream_t st) {
@@ -996,12 +1023,11 @@ void TsneDev::run(int n_iter, bool use_graph, cudaStream_t st) {
         }
         return;
     }
-    if (graph && graph_stream != st) { cudaGraphExecDestroy(graph); graph = nullptr; }
-    if (!graph) {
-        graph = capture_loop([&](cudaStream_t cap, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join) {
+    if (!graph || graph_stale) {
+        capture_loop([&](cudaStream_t cap, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join) {
             loop_iterate(a, z, &lanes, 1, cap, side, fork, join, nullptr);
-        }, graph_kernels);
-        graph_stream = st;
+        }, graph, graph_kernels);
+        graph_stale = false;
         graph_sig = signature();
     }
     for (int i = 0; i < n_iter; ++i) {
@@ -1011,10 +1037,12 @@ void TsneDev::run(int n_iter, bool use_graph, cudaStream_t st) {
     }
 }
 
-// one iteration captured on private streams (capture on the legacy default stream is not allowed); kernels = the
-// launches it holds (captured, not run: the replays count them)
-cudaGraphExec_t capture_loop(const std::function<void(cudaStream_t, cudaStream_t, cudaEvent_t, cudaEvent_t)>& body,
-                             uint64_t& kernels) {
+// One iteration captured on private streams (capture on the legacy default stream is not allowed) into `exec`; kernels =
+// the launches it holds (captured, not run: the replays count them). An executable that is there takes the new launches
+// (the nodes are the same kinds in the same order, unless a kernel's variant changed), which is quicker than
+// instantiating another; replays already under way are not affected.
+void capture_loop(const std::function<void(cudaStream_t, cudaStream_t, cudaEvent_t, cudaEvent_t)>& body,
+                  cudaGraphExec_t& exec, uint64_t& kernels) {
     struct Owned {
         cudaStream_t cap = nullptr, side = nullptr;
         cudaEvent_t fork = nullptr, join = nullptr;
@@ -1043,9 +1071,14 @@ cudaGraphExec_t capture_loop(const std::function<void(cudaStream_t, cudaStream_t
     kernels = launch_count() - before;
     count_launch(0 - kernels);
     MGB_CUDA(cudaStreamEndCapture(o.cap, &o.gr));
-    cudaGraphExec_t exec = nullptr;
+    if (exec) {
+        cudaGraphExecUpdateResultInfo info;
+        if (cudaGraphExecUpdate(exec, o.gr, &info) == cudaSuccess) return;
+        cudaGetLastError();
+        cudaGraphExecDestroy(exec);
+        exec = nullptr;
+    }
     MGB_CUDA(cudaGraphInstantiate(&exec, o.gr, 0));
-    return exec;
 }
 
 void TsneDev::run_profiled(int n_iter, cudaStream_t st, double* stage_ms, int* grid) {

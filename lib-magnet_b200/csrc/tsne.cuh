@@ -29,7 +29,7 @@ struct TsneDev {
     DevBuf Ycur, Ynext, U, G, ip, ix, P, gdesc, box_part, mean_part;
     RepBuffers rb;
     cudaGraphExec_t graph = nullptr;
-    cudaStream_t graph_stream = nullptr;
+    bool graph_stale = false;           // it was captured with another signature
     uint64_t graph_kernels = 0;         // kernel nodes of the captured iteration
     std::string graph_sig;              // sizes, schedule and buffer addresses the graph was captured with
     // spatial order of the points (the loop of a large layout): row r of every per-point array holds the caller's
@@ -39,9 +39,10 @@ struct TsneDev {
     int reorder_every = 0;              // iterations between reorders (0: never)
     DevBuf perm, perm_t, okey, ocnt, ostart, osrc, onew, olen, oip, oscan, Yt, Ut, Gt, ipt, ixt, Pt;
     ~TsneDev();
-    // P must already be normalised to sum 1 (done by the caller, as magnet/tsne.py:149-150)
-    void init(const int32_t* ip_h, const int32_t* ix_h, const float* P_h, int64_t n, int64_t nnz, bool host_ptrs,
-              const TsneSched& s, float dof, int threads_per_row, cudaStream_t st);
+    // sizes the buffers and copies the graph (device arrays); the caller then writes its affinities, normalised to sum 1
+    // (magnet/tsne.py:149-150), to P
+    void init(const int32_t* ip_d, const int32_t* ix_d, int64_t n, int64_t nnz, const TsneSched& s, float dof,
+              int threads_per_row, cudaStream_t st);
     void set_layout(const float* Y, bool host_ptr, cudaStream_t st);   // also resets update = 0, gains = 1
     void get_layout(float* Y, bool host_ptr, cudaStream_t st);         // applies the pending recentring
     LoopDesc desc();   // what the loop's kernels read
@@ -68,8 +69,8 @@ struct LaneRun {
 void loop_iterate(const LoopArgs& a, const LoopSizes& z, const LaneRun* runs, int n_runs, cudaStream_t st,
                   cudaStream_t side, cudaEvent_t fork, cudaEvent_t join, cudaEvent_t* ev);
 
-// a captured iteration: body(stream, side stream, fork, join) launches it
-cudaGraphExec_t capture_loop(const std::function<void(cudaStream_t, cudaStream_t, cudaEvent_t, cudaEvent_t)>& body,
-                             uint64_t& kernels);
+// a captured iteration: body(stream, side stream, fork, join) launches it; exec is made or brought up to it
+void capture_loop(const std::function<void(cudaStream_t, cudaStream_t, cudaEvent_t, cudaEvent_t)>& body,
+                  cudaGraphExec_t& exec, uint64_t& kernels);
 
 }  // namespace mgb
