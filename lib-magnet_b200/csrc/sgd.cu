@@ -9,8 +9,8 @@
 //    Negative p is draw p; the mid-range draws are draws 1024, 1025, ...; the distance-0 jitter of negative p
 //    in dimension d is draw 2048 + 64 p + d. Any lane can take any draw directly with one 32-bit hash, so the
 //    draws of a sample need no coordination. With the edges sorted by head (the reference's schedule is the COO of a
-//    sorted CSR) one thread owns a head row and applies the head's steps one after another, as the reference's
-//    loop does; the tails and partners move through hogwild float2 atomics. At most n / 8 rows are in flight.
+//    sorted CSR) one walker holds a head row and applies the head's steps one after another, as the reference's
+//    loop does; the tails and partners move through hogwild float2 atomics. At most n / 4 rows are in flight.
 //  * serial (stream_mode 1): the reference's single stream per epoch (n_threads = 1) is replayed exactly. The
 //    schedule (eons / eonns) is computed in parallel; one thread walks the sampled edges in order to find where
 //    each edge's draws start in the stream (its RNG state is recorded), then the head rows run in parallel from
@@ -26,6 +26,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <mutex>
+#include <type_traits>
 #include <unordered_map>
 
 namespace mgb {
@@ -350,10 +351,10 @@ __device__ __forceinline__ void flush_head(const SgdDev& c, int64_t u, int dim, 
 }
 
 // ---------------------------------------------------------------------------------------------- counter mode kernels
-// The counter mode's fast path (loss 0, dim 2 or 3, edges sorted by head) runs an epoch as three kernels (the split
-// form below): the epoch's sampled edges as a bit set with per-chunk counts, the counts' prefix sums, and the sample
-// pass, in which each thread walks an equal share of the samples in edge order. A sample first gathers what it
-// reads (tail, draws, the positions of its tail and negatives), then computes.
+// The counter mode's fast path (loss 0, dim 2 or 3, edges sorted by head): which edges an epoch samples, with how many
+// negatives, does not depend on the positions, so the samples of a batch of epochs are listed ahead (the list form
+// below), and an epoch is one pass over its list, in which each thread walks an equal share of the samples in edge
+// order, the next sample's positions under way while it computes.
 constexpr int kNegBatch = 6;   // n_neg is 4-6 for almost every sample (its long-run mean is the rate, 5)
 
 template <int D>
@@ -367,15 +368,20 @@ __device__ __forceinline__ void load_pos(const float* __restrict__ Y, int64_t k,
     }
 }
 
-// what a sample reads before it computes
+// A sample of the list: its draw key (or, of the thread form, its edge), head, tail and number of negatives
+struct alignas(16) Sample {
+    uint32_t key;
+    int32_t u, v, nn;
+};
+
+// what a sample reads before it computes; bit q of `live`: negative q exists and is not the head; w: its mid-range
+// partner (negative: none)
 template <int D>
 struct Fetched {
-    int64_t i;
+    uint32_t key, live;
     int nn;
-    int32_t v;
-    uint32_t key;
-    float yv[D];
-    int32_t k[kNegBatch];
+    int32_t v, w;
+    float yv[D], yw[D];
     float yk[kNegBatch][D];
 };
 
@@ -433,7 +439,7 @@ __device__ __forceinline__ void compute_sample(const SgdDev& c, int64_t u, const
     }
 #pragma unroll
     for (int q = 0; q < kNegBatch; ++q)
-        if (f.k[q] >= 0 && f.k[q] != (int32_t)u) add_negative<D, FAST, REP1>(c, u, yu, f.yk[q], f.key, q, jit, gu);
+        if (f.live >> q & 1u) add_negative<D, FAST, REP1>(c, u, yu, f.yk[q], f.key, q, jit, gu);
     for (int p = kNegBatch; p < f.nn; ++p) {   // rare: more negatives than one batch
         const int32_t k = (int32_t)below_of(counter_draw(f.key, p), (uint32_t)c.n);
         if (k == (int32_t)u) continue;
@@ -441,72 +447,100 @@ __device__ __forceinline__ void compute_sample(const SgdDev& c, int64_t u, const
         load_pos<D>(c.Y, k, yk);
         add_negative<D, FAST, REP1>(c, u, yu, yk, f.key, p, jit, gu);
     }
-    if (mid_w > 0.0f) {
-        CounterDraws dr(f.key);
-        if (uniform_of(dr.mid()) < c.mid_rate) {
-            const int32_t w = mid_partner(c, (int32_t)u, f.v, dr);
-            if (w != (int32_t)u) {
-                float yw[D], gk[D];
-                load_pos<D>(c.Y, w, yw);
+    if (f.w >= 0) {
+        float gk[D];
 #pragma unroll
-                for (int d = 0; d < D; ++d) { const float g = -mid_w * (yu[d] - yw[d]); gu[d] += g; gk[d] = -g; }
-                if (w >= c.n_fixed) HogwildSink().template apply<D>(c, w, gk, alpha, D);
-            }
-        }
+        for (int d = 0; d < D; ++d) { const float g = -mid_w * (yu[d] - f.yw[d]); gu[d] += g; gk[d] = -g; }
+        if (f.w >= c.n_fixed) HogwildSink().template apply<D>(c, f.w, gk, alpha, D);
     }
     if (u >= c.n_fixed) local_step<D>(c, yu, gu, alpha, u, D);
 }
 
-// One sample of the split form: the schedule update of its edge (eons / eonns as schedule_edge), then the sample's
-// reads and its steps. The reads that do not depend on one another (the edge's schedule state and tail) are issued
-// together, then the positions of the tail and the negatives.
-template <int D, bool FAST, bool REP1, bool B1>
-__device__ __forceinline__ void range_sample(const SgdDev& c, int64_t u, int64_t i, int epoch, float fepoch,
-                                             float alpha, float mid_w, float jit, float* yu) {
-    const float2 eo = c.eo[i];
-    const EdgeRO te = c.te[i];
-    const float eon = eo.x, eonn = eo.y, eps = te.eps;
-    const int32_t v = te.tail;
-    const uint32_t key = sample_key(stream_seed(c.seed, epoch, (uint64_t)i));
-    const float epn = eps / c.negative_sample_rate;
-    int nn = (int)((fepoch - eonn) / epn);
-    c.eo[i] = make_float2(__fadd_rn(eon, eps), __fadd_rn(eonn, __fmul_rn((float)nn, epn)));
-    nn = nn > 0 ? nn : 0;
-    Fetched<D> f;
-    f.i = i;
-    f.nn = nn;
-    f.v = v;
-    f.key = key;
-    load_pos<D>(c.Y, v, f.yv);
-#pragma unroll
-    for (int q = 0; q < kNegBatch; ++q) {
-        f.k[q] = q < nn ? (int32_t)below_of(counter_draw(key, q), (uint32_t)c.n) : -1;
-        if (f.k[q] >= 0) load_pos<D>(c.Y, f.k[q], f.yk[q]);
-    }
-    compute_sample<D, FAST, REP1, B1>(c, u, f, alpha, mid_w, jit, yu);
+__device__ __forceinline__ Sample load_sample(const Sample* p) {
+    const int4 v = __ldg(reinterpret_cast<const int4*>(p));
+    return Sample{(uint32_t)v.x, v.y, v.z, v.w};
 }
 
-// ---------------------------------------------------------------------------------------------- split form
-// The sample pass with the samples split evenly: thread t of T takes the samples of ranks [t S / T, (t + 1) S / T)
-// of the epoch's S sampled edges, in edge order, one sample per trip of its loop (so a warp's lanes stay converged
-// and carry equal counts). The edges are sorted by head, so a thread walks consecutive edges and a head's steps
-// follow one another in its registers as in the reference's loop; the head's displacement lands with one atomic
-// when the thread leaves the row (a row cut between two threads is held by both, and each lands its own). The
-// schedule update of a sampled edge (eons / eonns) happens once, in the sample that consumes it. The sampled set is
-// one bit per edge (eons <= epoch, the test of src/layout.cpp:135), counted per chunk of kChunkWords words, so a
-// thread finds its first sample by a binary search of the chunks' prefix sums and a walk of one chunk.
-constexpr int kChunkWords = 64;   // 2048 edges per chunk
-constexpr int kSplitBlock = 128;  // threads per block of the sample pass
+// the mid-range partner of a sample (src/layout.cpp:225-249), -1 where there is none
+__device__ __forceinline__ int32_t partner_of(const SgdDev& c, uint32_t key, int32_t u, int32_t v, float mid_w) {
+    if (!(mid_w > 0.0f)) return -1;
+    CounterDraws dr(key);
+    if (!(uniform_of(dr.mid()) < c.mid_rate)) return -1;
+    const int32_t w = mid_partner(c, u, v, dr);
+    return w != u ? w : -1;
+}
 
-// the chunks' exclusive prefix sums and, in cpre[n], the total: one block, each thread a run of consecutive
-// chunks (summed, then a block scan of the run sums, then the run written), so the scan waits on one round of loads
-// instead of one per 1024 chunks
+// the positions a sample reads, issued together
+template <int D>
+__device__ __forceinline__ void fetch_sample(const SgdDev& c, const Sample& r, int32_t w, Fetched<D>& f) {
+    f.key = r.key; f.nn = r.nn; f.v = r.v; f.w = w; f.live = 0u;
+    load_pos<D>(c.Y, r.v, f.yv);
+#pragma unroll
+    for (int q = 0; q < kNegBatch; ++q) {
+        const int32_t k = (int32_t)below_of(counter_draw(r.key, q), (uint32_t)c.n);
+        if (q < r.nn && k != r.u) {
+            f.live |= 1u << q;
+            load_pos<D>(c.Y, k, f.yk[q]);
+        }
+    }
+    if (w >= 0) load_pos<D>(c.Y, w, f.yw);
+}
+
+// ---------------------------------------------------------------------------------------------- list form
+// 1. list_count_kernel: per run of `words` x 32 edges (one warp) and epoch of the window, the number of samples (eons <=
+//    epoch, the test of src/layout.cpp:135, with eons advanced along the window).
+// 2. list_scan_kernel: per epoch, the runs' exclusive prefix sums and the total.
+// 3. list_emit_kernel: the schedule once more (eonns too), each epoch's samples written in edge order; eons / eonns
+//    advanced by the epochs of the batch.
+// 4. hogwild_list_kernel, per epoch: thread t of T takes samples [t S / T, (t + 1) S / T), one per trip of its loop (so a
+//    warp's lanes stay converged and carry equal counts). The edges are sorted by head, so a head's steps follow one
+//    another in the thread's registers as in the reference's loop; its displacement lands with one atomic when the
+//    thread leaves the row (a row cut between two threads is held by both, and each lands its own).
+//
+// Bound by latency in small layouts (T is n / 4, one warp per SM at 10,000 points) and by the rate of scattered 32-byte
+// reads in large ones. While the sample pass found its edges itself (a bit set, then the edge's schedule state, then
+// the positions, one after another, and a mid-range partner after those), an epoch took 100 us at 10,000 points and 456 us
+// at 1M; now 31 and 275, of which the lists take 1.4 and 80.
+constexpr int kSplitBlock = 128;  // threads per block of the sample pass
+constexpr int64_t kMaxWalkers = (int64_t)5 * kSplitBlock * kNumSMs;   // resident threads of the thread form
+constexpr int kWindow = 32;       // epochs counted together (one per lane)
+constexpr int kMaxWords = 64;     // words of 32 edges per run
+
+struct EpochBases {
+    int64_t at[kWindow];   // first sample of each of the batch's epochs
+};
+
+__global__ void __launch_bounds__(kThreads) list_count_kernel(const float* __restrict__ eons, const float* __restrict__ eps,
+                                                              int64_t E, int words, int64_t n_runs, int epoch0, int epochs,
+                                                              int64_t* __restrict__ count) {
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    for (int64_t run = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; run < n_runs; run += warps) {
+        int total = 0;   // of epoch `lane`
+        for (int w = 0; w < words; ++w) {
+            const int64_t i = (run * words + w) * 32 + lane;
+            float eon = i < E ? eons[i] : INFINITY;
+            const float ep = i < E ? eps[i] : 0.f;
+            for (int b = 0; b < epochs; ++b) {
+                const bool smp = !(eon > (float)(epoch0 + b));
+                const unsigned m = __ballot_sync(0xffffffffu, smp);
+                if (smp) eon = __fadd_rn(eon, ep);
+                if (lane == b) total += __popc(m);
+            }
+        }
+        if (lane < epochs) count[(int64_t)lane * n_runs + run] = total;
+    }
+}
+
+// epoch blockIdx.x: the runs' exclusive prefix sums, and the total; each thread a run of consecutive counts (summed,
+// then a block scan of the sums, then written)
 constexpr int kScanThreads = 1024;
-__global__ void __launch_bounds__(kScanThreads) chunk_scan_kernel(const int32_t* __restrict__ count, int64_t n,
-                                                                   int64_t* __restrict__ cpre) {
+__global__ void __launch_bounds__(kScanThreads) list_scan_kernel(int64_t* __restrict__ count, int64_t n_runs,
+                                                                  int64_t* __restrict__ totals) {
     __shared__ int64_t wsum[kScanThreads / 32];
-    const int64_t per = (n + blockDim.x - 1) / blockDim.x;
-    const int64_t b = (int64_t)threadIdx.x * per, e = b + per < n ? b + per : n;
+    count += (int64_t)blockIdx.x * n_runs;
+    const int64_t per = (n_runs + blockDim.x - 1) / blockDim.x;
+    const int64_t b = (int64_t)threadIdx.x * per, e = b + per < n_runs ? b + per : n_runs;
     int64_t run = 0;
     for (int64_t i = b; i < e; ++i) run += count[i];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -519,7 +553,7 @@ __global__ void __launch_bounds__(kScanThreads) chunk_scan_kernel(const int32_t*
     if (lane == 31) wsum[warp] = x;
     __syncthreads();
     if (warp == 0) {
-        int64_t w = lane < (int)(blockDim.x >> 5) ? wsum[lane] : 0;
+        int64_t w = wsum[lane];
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const int64_t y = __shfl_up_sync(0xffffffffu, w, o);
@@ -529,115 +563,221 @@ __global__ void __launch_bounds__(kScanThreads) chunk_scan_kernel(const int32_t*
     }
     __syncthreads();
     int64_t acc = x - run + (warp > 0 ? wsum[warp - 1] : 0);
-    for (int64_t i = b; i < e; ++i) { cpre[i] = acc; acc += count[i]; }
-    if (threadIdx.x == blockDim.x - 1) cpre[n] = acc;
+    for (int64_t i = b; i < e; ++i) { const int64_t n = count[i]; count[i] = acc; acc += n; }
+    if (threadIdx.x == blockDim.x - 1) totals[blockIdx.x] = acc;
 }
 
-// the bit set (bit i of bits[i / 32] set when edge i is sampled), one warp ballot per 32 edges and one warp per
-// chunk, and the chunk's count of sampled edges; words past the last edge are written as 0, so every chunk is whole
-__global__ void __launch_bounds__(kThreads) chunk_bits_kernel(const float2* __restrict__ eo, int64_t E, float fepoch,
-                                                              int64_t n_chunks, uint32_t* __restrict__ bits,
-                                                              int32_t* __restrict__ count) {
+template <bool KEYS>
+__global__ void __launch_bounds__(kThreads) list_emit_kernel(SgdDev c, int words, int64_t n_runs, int epoch0, int epochs,
+                                                             const int64_t* __restrict__ count,
+                                                             const __grid_constant__ EpochBases base,
+                                                             Sample* __restrict__ list) {
     const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t ch = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; ch < n_chunks; ch += warps) {
-        const int64_t base = ch * (kChunkWords * 32);
-        int total = 0;
-#pragma unroll 1
-        for (int w0 = 0; w0 < kChunkWords; w0 += 8) {
-            bool smp[8];
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const int64_t i = base + (int64_t)(w0 + q) * 32 + lane;
-                smp[q] = i < E && !(eo[i].x > fepoch);
+    for (int64_t run = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; run < n_runs; run += warps) {
+        int64_t at = lane < epochs ? base.at[lane] + count[(int64_t)lane * n_runs + run] : 0;   // of epoch `lane`
+        for (int w = 0; w < words; ++w) {
+            const int64_t i = (run * words + w) * 32 + lane;
+            const bool in = i < c.n_edges;
+            const float eon0 = in ? c.eons[i] : INFINITY;
+            const float ep = in ? c.eps[i] : 0.f;
+            float eon = eon0, eonn = in ? c.eonns[i] : 0.f;
+            const int32_t u = in ? c.head[i] : 0, v = in ? c.tail[i] : 0;
+            const float epn = ep / c.negative_sample_rate;
+            for (int b = 0; b < epochs; ++b) {
+                const float fepoch = (float)(epoch0 + b);
+                const bool smp = !(eon > fepoch);
+                const unsigned m = __ballot_sync(0xffffffffu, smp);
+                const int64_t first = __shfl_sync(0xffffffffu, at, b);
+                if (smp) {
+                    // the schedule of src/layout.cpp:135, 160-163
+                    eon = __fadd_rn(eon, ep);
+                    const int nn = (int)((fepoch - eonn) / epn);
+                    eonn = __fadd_rn(eonn, __fmul_rn((float)nn, epn));
+                    const uint32_t key = KEYS ? sample_key(stream_seed(c.seed, epoch0 + b, (uint64_t)i)) : (uint32_t)i;
+                    list[first + __popc(m & below)] = Sample{key, u, v, nn > 0 ? nn : 0};
+                }
+                if (lane == b) at += __popc(m);
             }
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const uint32_t m = __ballot_sync(0xffffffffu, smp[q]);
-                total += __popc(m);
-                if (lane == q) bits[ch * kChunkWords + w0 + q] = m;
-            }
+            if (in && !(eon0 > (float)(epoch0 + epochs - 1))) { c.eons[i] = eon; c.eonns[i] = eonn; }
         }
-        if (lane == 0) count[ch] = total;
     }
 }
 
-template <int D, bool FAST, bool REP1, bool B1>
-__global__ void __launch_bounds__(kThreads, 4) hogwild_split_kernel(SgdDev c, const int64_t* __restrict__ eptr,
-                                                                    const uint32_t* __restrict__ bits,
-                                                                    const int64_t* __restrict__ cpre, int64_t n_chunks,
-                                                                    int epoch, float alpha, float mid_w) {
-    const float fepoch = (float)epoch;
+template <int D, bool FAST, bool REP1, bool B1, bool AHEAD>
+__global__ void __launch_bounds__(kSplitBlock, D == 2 ? 5 : 4) hogwild_list_kernel(SgdDev c, const Sample* __restrict__ list, int64_t S,
+                                                                                   int epoch, float alpha, float mid_w) {
     const float jit = 1e-3f / fmaxf(alpha, 1e-6f);
     const int64_t T = (int64_t)gridDim.x * blockDim.x;
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t S = cpre[n_chunks];
     const int64_t r0 = t * S / T, r1 = (t + 1) * S / T;
     if (r0 >= r1) return;
-    // the chunk holding the sample of rank r0: the last chunk whose prefix is <= r0 (it has a sample past r0)
-    int64_t lo = 0, hi = n_chunks;
-    while (hi - lo > 1) {
-        const int64_t mid = (lo + hi) >> 1;
-        if (cpre[mid] <= r0) lo = mid; else hi = mid;
-    }
-    int64_t k = r0 - cpre[lo];
-    int64_t w = lo * kChunkWords;
-    const int64_t w_end = n_chunks * kChunkWords;
-    uint32_t m = bits[w];
-    while (k >= __popc(m) && w + 1 < w_end) { k -= __popc(m); m = bits[++w]; }
-    for (int j = 0; j < (int)k; ++j) m &= m - 1u;
-    if (m == 0u) return;   // counts and bits disagree: cannot happen, both come from one ballot
-    int64_t pos = w * 32 + __ffs(m) - 1;
-    const int64_t end = c.n_edges;
-    int64_t u = c.head[pos], row_end = eptr[u + 1];
+    // samples under way: r computes, the positions of r + 1 (AHEAD), the partner of the next one and the entry of the one
+    // after that are being read
+    auto entry = [&](int64_t r) {   // (past the end: the last one again, unused)
+        return load_sample(list + (r < r1 ? r : r1 - 1));
+    };
+    auto keyed = [&](Sample x) { x.key = sample_key(stream_seed(c.seed, epoch, (uint64_t)x.key)); return x; };
+    auto partner = [&](int64_t r, const Sample& x) { return r < r1 ? partner_of(c, x.key, x.u, x.v, mid_w) : -1; };
     float yu[D], y0[D];
-    bool have = false;
-    for (int64_t left = r1 - r0; left > 0; --left) {
-        int64_t i = -1;
-        while (pos < end) {
-            const uint32_t mm = bits[pos >> 5] & (0xffffffffu << (pos & 31));
-            if (mm) { i = (pos & ~(int64_t)31) + __ffs(mm) - 1; pos = i + 1; break; }
-            pos = (pos | 31) + 1;
-        }
-        if (i < 0 || i >= end) break;
-        if (i >= row_end) {
-            if (have && u >= c.n_fixed) flush_head<D>(c, u, D, yu, y0);
-            have = false;
-            do { ++u; row_end = eptr[u + 1]; } while (i >= row_end);
-        }
-        if (!have) {
-            load_pos<D>(c.Y, u, yu);
+    Fetched<D> cur;
+    Sample next = keyed(entry(r0));
+    int32_t u = next.u, w = partner(r0, next);
+    Sample after = keyed(entry(r0 + 1)), third = entry(r0 + 2);
+    load_pos<D>(c.Y, u, yu);
 #pragma unroll
-            for (int d = 0; d < D; ++d) y0[d] = yu[d];
-            have = true;
+    for (int d = 0; d < D; ++d) y0[d] = yu[d];
+    if constexpr (AHEAD) {
+        fetch_sample<D>(c, next, w, cur);
+        next = after;
+        w = partner(r0 + 1, next);
+    }
+    for (int64_t r = r0; r < r1; ++r) {
+        if constexpr (AHEAD) {
+            Fetched<D> ahead;
+            float yh[D];
+            after = keyed(third);
+            third = entry(r + 3);
+            const int32_t un = next.u;
+            const bool more = r + 1 < r1, leave = more && un != u;
+            if (leave) load_pos<D>(c.Y, un, yh);
+            if (more) fetch_sample<D>(c, next, w, ahead);
+            w = partner(r + 2, after);
+            next = after;
+            compute_sample<D, FAST, REP1, B1>(c, u, cur, alpha, mid_w, jit, yu);
+            if (leave) {
+                if (u >= c.n_fixed) flush_head<D>(c, u, D, yu, y0);
+#pragma unroll
+                for (int d = 0; d < D; ++d) { yu[d] = yh[d]; y0[d] = yh[d]; }
+                u = un;
+            }
+            if (more) cur = ahead;
+        } else {
+            fetch_sample<D>(c, next, w, cur);
+            w = partner(r + 1, after);
+            next = after;
+            after = keyed(third);
+            third = entry(r + 3);
+            compute_sample<D, FAST, REP1, B1>(c, u, cur, alpha, mid_w, jit, yu);
+            if (r + 1 < r1 && next.u != u) {
+                if (u >= c.n_fixed) flush_head<D>(c, u, D, yu, y0);
+                u = next.u;
+                load_pos<D>(c.Y, u, yu);
+#pragma unroll
+                for (int d = 0; d < D; ++d) y0[d] = yu[d];
+            }
         }
-        range_sample<D, FAST, REP1, B1>(c, u, i, epoch, fepoch, alpha, mid_w, jit, yu);
     }
-    if (have && u >= c.n_fixed) flush_head<D>(c, u, D, yu, y0);
+    if (u >= c.n_fixed) flush_head<D>(c, u, D, yu, y0);
 }
 
-// The split form's packed copies of the edge fields, made at the start of a call and (eons, eonns) written back at
-// its end; a sample then reads two records instead of four arrays and writes one.
-__global__ void pack_edges_kernel(const float* __restrict__ eons, const float* __restrict__ eonns,
-                                  const int32_t* __restrict__ tail, const float* __restrict__ eps, int64_t E,
-                                  float2* __restrict__ eo, EdgeRO* __restrict__ te) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < E; i += (int64_t)gridDim.x * blockDim.x) {
-        eo[i] = make_float2(eons[i], eonns[i]);
-        te[i] = EdgeRO{tail[i], eps[i]};
-    }
-}
-
-__global__ void unpack_edges_kernel(const float2* __restrict__ eo, int64_t E, float* __restrict__ eons,
-                                    float* __restrict__ eonns) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < E; i += (int64_t)gridDim.x * blockDim.x) {
-        const float2 v = eo[i];
-        eons[i] = v.x;
-        eonns[i] = v.y;
+// Small layouts: eight lanes per walker, one slot of the sample each (0 its tail, 1 to 6 its negatives, 7 its mid-range
+// partner), one position and one coefficient per lane, summed by shuffles. Every lane holds the head's position and takes its
+// step, the same arithmetic in each. Bound by the latency of its instructions (about nine cycles each with one warp per
+// scheduler), so the lanes' paths are one: positions are read whether needed or not, the coefficients share one
+// expression, and a warp's four walkers run the same number of trips (a finished one has no live slots). Plain SGD only
+// (Adam's state has one writer per step).
+constexpr int kLanes = 8;
+template <int D, bool FAST>
+__global__ void __launch_bounds__(kSplitBlock) hogwild_group_kernel(SgdDev c, const Sample* __restrict__ list, int64_t S,
+                                                                    int64_t T, float alpha, float mid_w) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const float jit = 1e-3f / fmaxf(alpha, 1e-6f);
+    const int j = threadIdx.x & (kLanes - 1);
+    const bool tail = j == 0, neg = j >= 1 && j <= kNegBatch, mid = j == kLanes - 1;
+    const int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kLanes;
+    const int64_t r0 = t < T ? t * S / T : 0;
+    const int count = t < T ? (int)((t + 1) * S / T - r0) : 0;
+    const int trips = __reduce_max_sync(kAll, count);
+    if (trips == 0) return;
+    const int last = max(count - 1, 0);
+    const float sa = tail ? c.a : c.rep_a, sb = tail ? c.b : c.rep_b, near = tail ? 0.0f : 0.001f;
+    const float attract = -c.exaggeration * 2.0f * c.a * c.b;
+    const bool one = tail ? c.b_is_one : c.rep_b_is_one;
+    const uint32_t draw = (uint32_t)(j - 1) * 0x9E3779B9u;
+    list += r0;
+    // the position of this lane's slot (w: the partner, in its lane), and whether the slot counts
+    auto fetch = [&](const Sample& x, int32_t w, float* p) {
+        int32_t k = tail ? x.v : x.u;
+        if (neg) k = (int32_t)__umulhi(hash32(x.key + draw), (uint32_t)c.n);   // below_of(counter_draw(key, j - 1), n)
+        if (mid && w >= 0) k = w;
+        load_pos<D>(c.Y, k, p);
+        return tail || (neg ? j - 1 < x.nn && k != x.u : w >= 0);
+    };
+    // the partner of r + 1 and the entry of r + 2 are being read while r computes
+    Sample cur = load_sample(list), next = load_sample(list + min(1, last));
+    int32_t w = mid ? partner_of(c, cur.key, cur.u, cur.v, mid_w) : -1;
+    float yu[D], y0[D], pos[D];
+    bool enter = true;   // the head's first sample here
+    for (int r = 0; r < trips; ++r) {
+        float yh[D];
+        load_pos<D>(c.Y, cur.u, yh);
+        const bool live = fetch(cur, w, pos) && r < count;
+        const Sample after = load_sample(list + min(r + 2, last));
+        const int32_t wn = mid ? partner_of(c, next.key, next.u, next.v, mid_w) : -1;
+        if (enter) {
+#pragma unroll
+            for (int d = 0; d < D; ++d) { yu[d] = yh[d]; y0[d] = yh[d]; }
+        }
+        float diff[D], gu[D], dd = 0.0f;
+#pragma unroll
+        for (int d = 0; d < D; ++d) { diff[d] = yu[d] - pos[d]; dd = __fadd_rn(dd, __fmul_rn(diff[d], diff[d])); }
+        float coeff = 0.0f;
+        if constexpr (FAST) {   // attraction and repulsion in one expression (compute_sample's and add_negative's)
+            const float pw = one ? dd : exp2f(sb * __log2f(dd));
+            coeff = mid ? -mid_w : __fdividef(tail ? attract * pw : c.two_b, (near + dd) * (sa * pw + 1.0f));
+        } else if (live && dd > 0.0f) {
+            if (mid) {
+                coeff = -mid_w;
+            } else if (tail) {
+                const float b_uv = c.node_b ? 0.5f * (c.node_b[cur.u] + c.node_b[cur.v]) : c.b;
+                coeff = attraction_coeff(c, dd, b_uv, (c.b_is_one && !c.node_b) ? dd : powf(dd, b_uv));
+            } else {
+                coeff = repulsion_coeff(c, dd, cur.u);
+            }
+        }
+        const bool moves = live && dd > 0.0f;
+#pragma unroll
+        for (int d = 0; d < D; ++d) gu[d] = moves ? coeff * diff[d] : 0.0f;
+        const int32_t other = tail ? cur.v : w;
+        if (!neg && moves && other >= c.n_fixed) {
+            float gk[D];
+#pragma unroll
+            for (int d = 0; d < D; ++d) gk[d] = -gu[d];
+            HogwildSink().template apply<D>(c, other, gk, alpha, D);
+        }
+        // rare: a negative on the head, more than six negatives
+        if (live && !moves && neg) {
+#pragma unroll
+            for (int d = 0; d < D; ++d)
+                gu[d] += (uniform_of(counter_draw(cur.key, kJitterDraw + 64 * (j - 1) + d)) - 0.5f) * jit;
+        }
+        if (r < count) {
+            for (int p = kNegBatch + j; p < cur.nn; p += kLanes) {
+                const int32_t k = (int32_t)below_of(counter_draw(cur.key, p), (uint32_t)c.n);
+                if (k == cur.u) continue;
+                float yk[D];
+                load_pos<D>(c.Y, k, yk);
+                if (FAST && c.rep_b_is_one) add_negative<D, FAST, true>(c, cur.u, yu, yk, cur.key, p, jit, gu);
+                else add_negative<D, FAST, false>(c, cur.u, yu, yk, cur.key, p, jit, gu);
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int o = kLanes / 2; o > 0; o >>= 1)
+#pragma unroll
+            for (int d = 0; d < D; ++d) gu[d] += __shfl_xor_sync(kAll, gu[d], o, kLanes);
+        if (r < count && cur.u >= c.n_fixed) local_step<D>(c, yu, gu, alpha, cur.u, D);
+        // the head's last sample here (past the walker's end every trip enters the last row again and leaves it unmoved)
+        enter = r + 1 >= count || next.u != cur.u;
+        if (enter && r < count && tail && cur.u >= c.n_fixed) flush_head<D>(c, cur.u, D, yu, y0);
+        cur = next; next = after; w = wn;
     }
 }
 
 // Blocks of a kernel the device holds at once (the SM count times the blocks one SM holds), asked once per kernel.
-// The split form's grid stays within it, so that no block waits for a second wave.
+// The list form's grid stays within it, so that no block waits for a second wave.
 template <typename K>
 int resident_blocks(K kernel) {
     static std::mutex mu;
@@ -648,7 +788,7 @@ int resident_blocks(K kernel) {
     int dev = 0, sms = 0, per_sm = 0;
     MGB_CUDA(cudaGetDevice(&dev));
     MGB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    MGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, 0));
+    MGB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kSplitBlock, 0));
     const int count = std::max(1, sms * per_sm);
     known.emplace(reinterpret_cast<const void*>(kernel), count);
     return count;
@@ -656,29 +796,44 @@ int resident_blocks(K kernel) {
 
 int env_int(const char* name, int dflt);
 
+// Lanes per walker: eight up to one and a half waves of them (nine blocks per SM; about 85,000 points), above, where the
+// thread form's warps hide each other's latency, one. us per epoch with one and with eight: 3,000 points 59 and 31, 10,000
+// 64 and 31, 47,000 72 and 42, 90,000 83 and 77, 200,000 102 and 146.
+int walker_lanes(const SgdDev& c, int64_t threads) {
+    if (c.optimizer == 1) return 1;
+    return threads * kLanes <= (int64_t)9 * kSplitBlock * kNumSMs ? kLanes : 1;
+}
+
 template <int D, bool FAST>
-void launch_split(const SgdDev& c, int64_t threads, const int64_t* eptr, uint32_t* bits, int32_t* count, int64_t* cpre,
-                  int64_t n_chunks, int epoch, float alpha, float mid_w, cudaStream_t s) {
-    chunk_bits_kernel<<<blocks_for(n_chunks * 32, kThreads, 8), kThreads, 0, s>>>(c.eo, c.n_edges, (float)epoch,
-                                                                                  n_chunks, bits, count);
-    MGB_LAUNCH_CHECK();
-    chunk_scan_kernel<<<1, kScanThreads, 0, s>>>(count, n_chunks, cpre);
-    MGB_LAUNCH_CHECK();
+void launch_list(const SgdDev& c, int64_t threads, int lanes, const Sample* list, int64_t S, int epoch, float alpha,
+                 float mid_w, cudaStream_t s) {
+    if (lanes > 1) {
+        const int64_t all = threads * lanes;
+        const int tpb = (int)std::min<int64_t>(kSplitBlock, std::max<int64_t>(32, (all / kNumSMs) / 32 * 32));
+        hogwild_group_kernel<D, FAST><<<(int)((all + tpb - 1) / tpb), tpb, 0, s>>>(c, list, S, threads, alpha, mid_w);
+        return;
+    }
     const bool rep1 = FAST && c.rep_b_is_one, b1 = FAST && c.b_is_one;
-    auto kernel = rep1 && b1 ? hogwild_split_kernel<D, FAST, true, true>
-                : rep1       ? hogwild_split_kernel<D, FAST, true, false>
-                : b1         ? hogwild_split_kernel<D, FAST, false, true>
-                             : hogwild_split_kernel<D, FAST, false, false>;
-    // blocks of 128 threads (0.439 ms per epoch at 1M points against 0.449 with 256: 640 blocks spread more evenly
-    // over the SMs than 320); few threads (small layouts): blocks of fewer threads, so that they reach every SM.
-    // MGB_SGD_BLOCK sets another block size.
-    int tpb = std::min(kThreads, std::max(32, env_int("MGB_SGD_BLOCK", kSplitBlock) / 32 * 32));
+    // Positions a sample ahead double what is in flight, so only where that stays within n / 4 (the walkers' own bound):
+    // 1M points 275 us an epoch with, 301 without (200,000, outside the bound: 85 and 102); 600-point layouts with it lost
+    // up to half a point of purity. Not with Adam.
+    const bool ahead = c.optimizer != 1 && 8 * threads <= c.n;
+    auto pick = [&](auto a) {
+        constexpr bool A = decltype(a)::value;
+        return rep1 && b1 ? hogwild_list_kernel<D, FAST, true, true, A>
+             : rep1       ? hogwild_list_kernel<D, FAST, true, false, A>
+             : b1         ? hogwild_list_kernel<D, FAST, false, true, A>
+                          : hogwild_list_kernel<D, FAST, false, false, A>;
+    };
+    auto kernel = ahead ? pick(std::true_type{}) : pick(std::false_type{});
+    // few threads (small layouts): blocks of fewer threads, so that they reach every SM. MGB_SGD_BLOCK sets another
+    // block size.
+    int tpb = std::min(kSplitBlock, std::max(32, env_int("MGB_SGD_BLOCK", kSplitBlock) / 32 * 32));
     if (threads < (int64_t)kNumSMs * tpb)
-        tpb = (int)std::min<int64_t>(kThreads, std::max<int64_t>(32, ((threads + kNumSMs - 1) / kNumSMs + 31) / 32 * 32));
+        tpb = (int)std::min<int64_t>(kSplitBlock, std::max<int64_t>(32, ((threads + kNumSMs - 1) / kNumSMs + 31) / 32 * 32));
     int64_t blocks = std::max<int64_t>(1, (threads + tpb - 1) / tpb);
-    if (tpb == kThreads) blocks = std::min<int64_t>(blocks, resident_blocks(kernel));
-    else blocks = std::min<int64_t>(blocks, (int64_t)resident_blocks(kernel) * (kThreads / tpb));
-    kernel<<<(int)blocks, tpb, 0, s>>>(c, eptr, bits, cpre, n_chunks, epoch, alpha, mid_w);
+    blocks = std::min<int64_t>(blocks, (int64_t)resident_blocks(kernel) * (kSplitBlock / tpb));
+    kernel<<<(int)blocks, tpb, 0, s>>>(c, list, S, epoch, alpha, mid_w);
 }
 
 // Row kernel (any dim, any loss): one thread owns a head row and walks it in order with counter draws.
@@ -834,8 +989,16 @@ __global__ void row_ptr_kernel(const int32_t* __restrict__ head, int64_t E, int6
 }
 
 __global__ void unsorted_kernel(const int32_t* __restrict__ head, int64_t E, int* __restrict__ flag) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x + 1; i < E; i += (int64_t)gridDim.x * blockDim.x)
-        if (head[i] < head[i - 1]) { *flag = 1; return; }
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x + 1; i < E; i += 4 * stride) {
+        bool falls = false;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {   // reads under way together
+            const int64_t k = i + q * stride;
+            if (k < E) falls |= head[k] < head[k - 1];
+        }
+        if (falls) { *flag = 1; return; }
+    }
 }
 
 // schedule hook: the draws of one epoch (no updates)
@@ -905,33 +1068,23 @@ int64_t max_in_flight(const SgdDev& c) {
     return std::max<int64_t>(64, c.n / div);
 }
 
-// Threads of the split form, each holding one head at a time: n / 4 (n / 8 with Adam, whose per-node moments take
+// Walkers of the list form, each holding one head at a time: n / 4 (n / 8 with Adam, whose per-node moments take
 // the concurrent steps of every thread that holds the node: at n / 4 a 600-point Adam layout lost 20 points of
-// neighbourhood purity), at most 81,920 (2.2 blocks of 256 per SM).
-// Measured on B200 (ms per epoch; 15-NN preservation of the finished layout unchanged within 0.002):
-// 1M points 0.485 at 83k threads, 0.51 at 125k, 0.53 at 167k; the 10k-point umap pass 53 ms at
-// n / 4, 94 ms at n / 8, 152 ms at n / 16 for 500 epochs. MGB_SGD_INFLIGHT_DIV = k sets n / k instead.
-constexpr int64_t kSplitMaxThreads = 81920;
+// neighbourhood purity), at most five blocks of 128 threads per SM (what the thread form keeps resident).
+// Measured on B200 (us per epoch; 15-NN preservation of the finished layout unchanged within 0.002): 1M points 312 with
+// 81,920 walkers, 292 with 94,720; the last tenth of a 10k-point umap pass 36 at n / 4, 61 at n / 8, 111 at n / 16, all
+// three with an earlier form of the passes.
+// MGB_SGD_INFLIGHT_DIV = k sets n / k instead.
 int64_t split_threads(const SgdDev& c) {
     const int div = env_int("MGB_SGD_INFLIGHT_DIV", 0);
     if (div > 0) return std::max<int64_t>(64, c.n / div);
-    return std::max<int64_t>(64, std::min<int64_t>(c.n / (c.optimizer == 1 ? 8 : 4), kSplitMaxThreads));
+    return std::max<int64_t>(64, std::min<int64_t>(c.n / (c.optimizer == 1 ? 8 : 4), kMaxWalkers));
 }
 
 template <int D>
-void hogwild_epoch(const SgdDev& c, SgdWork& w, const int64_t* eptr, int epoch, float alpha, float mid_w,
-                   cudaStream_t s) {
+void hogwild_epoch(const SgdDev& c, const int64_t* eptr, int epoch, float alpha, float mid_w, cudaStream_t s) {
     const int64_t cap = max_in_flight(c);
-    if (c.eo && eptr && c.loss == 0 && (D == 2 || D == 3)) {
-        const int64_t n_chunks = std::max<int64_t>(1, (c.n_edges + kChunkWords * 32 - 1) / (kChunkWords * 32));
-        uint32_t* bits = w.samp.as<uint32_t>();
-        int64_t* cpre = reinterpret_cast<int64_t*>(bits + n_chunks * kChunkWords);
-        int32_t* count = reinterpret_cast<int32_t*>(cpre + n_chunks + 1);
-        constexpr int DD = D == 0 ? 2 : D;
-        const int64_t threads = split_threads(c);
-        if (c.kernel == 0 && !c.node_b) launch_split<DD, true>(c, threads, eptr, bits, count, cpre, n_chunks, epoch, alpha, mid_w, s);
-        else launch_split<DD, false>(c, threads, eptr, bits, count, cpre, n_chunks, epoch, alpha, mid_w, s);
-    } else if (eptr) {
+    if (eptr) {
         const int blocks = (int)std::min<int64_t>(blocks_for(c.n, kThreads), (cap + kThreads - 1) / kThreads);
         hogwild_rows_kernel<D><<<blocks, kThreads, 0, s>>>(c, eptr, epoch, alpha, mid_w);
     } else {
@@ -964,9 +1117,8 @@ void record_launch(const SgdDev& c, int epoch, float alpha, float mid_w, const i
     record_kernel<D><<<blocks_for(c.n_edges, kThreads), kThreads, 0, s>>>(c, epoch, alpha, mid_w, cnt, st, per_edge, rec);
 }
 
-// row pointers when the edges are sorted by head, else nullptr (edge-parallel kernels)
-const int64_t* row_pointers(const SgdDev& c, SgdWork& w, cudaStream_t s) {
-    if (c.n_edges == 0) return nullptr;
+bool sorted_by_head(const SgdDev& c, SgdWork& w, cudaStream_t s) {
+    if (c.n_edges == 0) return false;
     int* flag = static_cast<int*>(w.flag.ensure(sizeof(int)));
     MGB_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), s));
     unsorted_kernel<<<blocks_for(c.n_edges, kThreads, 4), kThreads, 0, s>>>(c.head, c.n_edges, flag);
@@ -974,7 +1126,12 @@ const int64_t* row_pointers(const SgdDev& c, SgdWork& w, cudaStream_t s) {
     int h = 0;
     MGB_CUDA(cudaMemcpyAsync(&h, flag, sizeof(int), cudaMemcpyDeviceToHost, s));
     MGB_CUDA(cudaStreamSynchronize(s));
-    if (h) return nullptr;
+    return h == 0;
+}
+
+// row pointers when the edges are sorted by head, else nullptr (edge-parallel kernels)
+const int64_t* row_pointers(const SgdDev& c, SgdWork& w, bool sorted, cudaStream_t s) {
+    if (!sorted) return nullptr;
     int64_t* eptr = static_cast<int64_t*>(w.eptr.ensure(sizeof(int64_t) * (c.n + 1)));
     row_ptr_kernel<<<blocks_for(c.n + 1, kThreads, 4), kThreads, 0, s>>>(c.head, c.n_edges, c.n, eptr);
     MGB_LAUNCH_CHECK();
@@ -992,37 +1149,91 @@ void sgd_sched(const SgdDev& c, int epoch, int e0, int e1, float alpha0, float a
     mid_w = c.use_mid ? mid_w0 + (mid_w1 - mid_w0) * frac : 0.0f;
 }
 
+namespace {
+// The list form over epochs [e0, e1): batches of at most kWindow epochs whose samples fit the list, which holds twice the
+// edges (two full epochs; at least 4 million) unless one epoch needs more. The window after a batch is counted before
+// the batch's passes, so the host knows its totals while those run. (An epoch of a long schedule samples a quarter of the
+// edges or less, so the first window is four times what the list would hold of full epochs.)
+void run_lists(const SgdDev& c, SgdWork& w, int e0, int e1, float alpha0, float alpha1, float mid_w0, float mid_w1,
+               cudaStream_t s) {
+    // runs short enough that the warps fill the device, long enough that the counts stay few
+    const int64_t all_words = (c.n_edges + 31) / 32;
+    const int words = (int)std::max<int64_t>(1, std::min<int64_t>(kMaxWords, all_words / (kNumSMs * 32)));
+    const int64_t n_runs = (all_words + words - 1) / words;
+    int64_t* totals = static_cast<int64_t*>(w.samp.ensure(sizeof(int64_t) * kWindow * (n_runs + 1)));
+    int64_t* count = totals + kWindow;
+    const int64_t room = std::max({c.n_edges, std::min<int64_t>(2 * c.n_edges, (int64_t)1 << 26), (int64_t)1 << 22});
+    const int blocks = blocks_for(n_runs * 32, kThreads, 8);
+    w.host_totals(kWindow);
+    int window = 0;
+    auto count_window = [&](int e, int most) {
+        const int epochs = window = std::min(most, e1 - e);
+        list_count_kernel<<<blocks, kThreads, 0, s>>>(c.eons, c.eps, c.n_edges, words, n_runs, e, epochs, count);
+        MGB_LAUNCH_CHECK();
+        list_scan_kernel<<<epochs, kScanThreads, 0, s>>>(count, n_runs, totals);
+        MGB_LAUNCH_CHECK();
+        MGB_CUDA(cudaMemcpyAsync(w.totals, totals, sizeof(int64_t) * epochs, cudaMemcpyDeviceToHost, s));
+        MGB_CUDA(cudaEventRecord(w.counted, s));
+    };
+    const int64_t threads = split_threads(c);
+    const int lanes = walker_lanes(c, threads);
+    count_window(e0, (int)std::min<int64_t>(kWindow, 4 * room / c.n_edges));
+    for (int e = e0; e < e1;) {
+        MGB_CUDA(cudaEventSynchronize(w.counted));
+        int64_t S[kWindow];
+        EpochBases bases{};
+        int epochs = 0;
+        int64_t sum = 0;
+        while (epochs < window && (epochs == 0 || sum + w.totals[epochs] <= room)) {
+            S[epochs] = w.totals[epochs];
+            bases.at[epochs] = sum;
+            sum += S[epochs++];
+        }
+        if (w.list.bytes < sizeof(Sample) * (size_t)sum)
+            w.list.ensure(sizeof(Sample) * (size_t)std::max<int64_t>(sum, std::min<int64_t>(sum + sum / 4, room)));
+        Sample* list = w.list.as<Sample>();
+        auto emit = lanes > 1 ? list_emit_kernel<true> : list_emit_kernel<false>;
+        emit<<<blocks, kThreads, 0, s>>>(c, words, n_runs, e, epochs, count, bases, list);
+        MGB_LAUNCH_CHECK();
+        if (e + epochs < e1) count_window(e + epochs, epochs < window ? epochs + 1 : kWindow);
+        for (int b = 0; b < epochs; ++b) {
+            if (S[b] == 0) continue;
+            float alpha, mid_w;
+            sgd_sched(c, e + b, e0, e1, alpha0, alpha1, mid_w0, mid_w1, alpha, mid_w);
+            const bool fast = c.kernel == 0 && !c.node_b;
+            const Sample* l = list + bases.at[b];
+            if (c.dim == 2) {
+                if (fast) launch_list<2, true>(c, threads, lanes, l, S[b], e + b, alpha, mid_w, s);
+                else launch_list<2, false>(c, threads, lanes, l, S[b], e + b, alpha, mid_w, s);
+            } else {
+                if (fast) launch_list<3, true>(c, threads, lanes, l, S[b], e + b, alpha, mid_w, s);
+                else launch_list<3, false>(c, threads, lanes, l, S[b], e + b, alpha, mid_w, s);
+            }
+            MGB_LAUNCH_CHECK();
+        }
+        e += epochs;
+    }
+}
+}  // namespace
+
 void sgd_run(SgdDev& c, SgdWork& w, int stream_mode, int e0, int e1, float alpha0, float alpha1, float mid_w0,
              float mid_w1, cudaStream_t s) {
-    const int64_t* eptr = row_pointers(c, w, s);
+    const bool sorted = sorted_by_head(c, w, s);
     if (stream_mode == 0) {
-        SgdDev cc = c;
-        const bool split = eptr && c.loss == 0 && (c.dim == 2 || c.dim == 3) && c.n_edges > 0 && e1 > e0;
-        if (split) {
-            // the split form's bit per edge (whole chunks of 2048 edges), the chunks' prefix sums and counts, and
-            // the packed edge fields
-            const size_t n_chunks = (size_t)std::max<int64_t>(1, (c.n_edges + kChunkWords * 32 - 1) / (kChunkWords * 32));
-            w.samp.ensure(sizeof(uint32_t) * n_chunks * kChunkWords + sizeof(int64_t) * (n_chunks + 1) +
-                          sizeof(int32_t) * n_chunks);
-            char* pk = static_cast<char*>(w.pack.ensure((sizeof(float2) + sizeof(EdgeRO)) * (size_t)c.n_edges));
-            cc.eo = reinterpret_cast<float2*>(pk);
-            cc.te = reinterpret_cast<const EdgeRO*>(pk + sizeof(float2) * (size_t)c.n_edges);
-            pack_edges_kernel<<<blocks_for(c.n_edges, kThreads), kThreads, 0, s>>>(
-                c.eons, c.eonns, c.tail, c.eps, c.n_edges, cc.eo, const_cast<EdgeRO*>(cc.te));
-            MGB_LAUNCH_CHECK();
+        if (sorted && c.loss == 0 && (c.dim == 2 || c.dim == 3) && e1 > e0 && c.n_edges <= (int64_t)UINT32_MAX) {
+            run_lists(c, w, e0, e1, alpha0, alpha1, mid_w0, mid_w1, s);
+            return;
         }
+        const int64_t* eptr = row_pointers(c, w, sorted, s);
         for (int e = e0; e < e1; ++e) {
             float alpha, mid_w;
-            sgd_sched(cc, e, e0, e1, alpha0, alpha1, mid_w0, mid_w1, alpha, mid_w);
-            MGB_DIM_DISPATCH(cc.dim, hogwild_epoch, cc, w, eptr, e, alpha, mid_w, s);
-            MGB_LAUNCH_CHECK();
-        }
-        if (split) {
-            unpack_edges_kernel<<<blocks_for(c.n_edges, kThreads), kThreads, 0, s>>>(cc.eo, c.n_edges, c.eons, c.eonns);
+            sgd_sched(c, e, e0, e1, alpha0, alpha1, mid_w0, mid_w1, alpha, mid_w);
+            MGB_DIM_DISPATCH(c.dim, hogwild_epoch, c, eptr, e, alpha, mid_w, s);
             MGB_LAUNCH_CHECK();
         }
         return;
     }
+    const int64_t* eptr = row_pointers(c, w, sorted, s);
     int32_t* cnt = static_cast<int32_t*>(w.cnt.ensure(sizeof(int32_t) * std::max<int64_t>(c.n_edges, 1)));
     uint64_t* st = static_cast<uint64_t*>(w.state.ensure(sizeof(uint64_t) * std::max<int64_t>(c.n_edges, 1)));
     const int64_t total = c.n * c.dim;

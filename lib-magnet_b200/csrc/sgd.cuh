@@ -4,12 +4,6 @@
 
 namespace mgb {
 
-// An edge's read-only fields, packed for the split form (one 8-byte load per sample)
-struct alignas(8) EdgeRO {
-    int32_t tail;
-    float eps;
-};
-
 // Everything an epoch kernel reads (the reference's Ctx, src/layout.cpp:69-88), as device pointers plus the
 // scalars derived once per call (src/layout.cpp:421-431).
 struct SgdDev {
@@ -26,9 +20,6 @@ struct SgdDev {
     const float* node_b;
     float* adam_m; float* adam_v; int32_t* adam_t; float beta1, beta2;
     uint64_t seed;
-    // the split form's packed copies for one call: (eons, eonns) per edge, and (tail, eps) per edge
-    float2* eo = nullptr;
-    const EdgeRO* te = nullptr;
 };
 
 // launches F<2>, F<3> or the generic F<0> (dims up to kMaxDim) for a layout of `dim` columns
@@ -42,12 +33,22 @@ struct SgdDev {
 // device scratch of the stream modes and of owner mode
 struct SgdWork {
     DevBuf cnt, state, delta, eptr, flag;
-    DevBuf samp;               // the epoch's sampled set (counter mode fast path)
-    DevBuf pack;               // the split form's packed edge fields
+    // counter mode's fast path: a window's counts of samples, the batch's samples, the totals on the host
+    DevBuf samp, list;
+    int64_t* totals = nullptr;
+    cudaEvent_t counted = nullptr;
+    void host_totals(int count) {
+        if (!totals) MGB_CUDA(cudaMallocHost(reinterpret_cast<void**>(&totals), sizeof(int64_t) * count));
+        if (!counted) MGB_CUDA(cudaEventCreateWithFlags(&counted, cudaEventDisableTiming));
+    }
     // owner mode: node rows, chunk bounds, per epoch and edge the negatives and head states, marked chunks, copies
     // of the layout and the Adam state, the barrier and head count, the list of heads
     DevBuf o_row, o_own, o_neg, o_state, o_dirty, o_snap, o_snap_m, o_snap_v, o_snap_t, o_sync, o_heads;
     bool flags_ready = false;  // flag[1] (a grid barrier gave up) has been cleared once
+    ~SgdWork() {
+        if (totals) cudaFreeHost(totals);
+        if (counted) cudaEventDestroy(counted);
+    }
 };
 
 void sgd_sched(const SgdDev& c, int epoch, int e0, int e1, float alpha0, float alpha1, float mid_w0, float mid_w1,
