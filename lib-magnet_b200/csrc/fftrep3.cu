@@ -444,6 +444,7 @@ __global__ void __launch_bounds__(kRowThreads, kRowBlocks) row_inv3_kernel(const
                 for (int q = 0; q < nbuf; ++q) {
                     const float4 v = src[q];
                     float2 x = make_float2(v.x, v.y), y = make_float2(v.z, v.w);
+                    if (g0 + 2 * q + 1 >= N) y = make_float2(0.f, 0.f);   // no row b: nothing was written there
                     if (kk == 0 || (even && kk == M / 2)) { x.y = 0.f; y.y = 0.f; }
                     if (k >= Mh) { x.y = -x.y; y.y = -y.y; }
                     (q ? B : A)[pos] = make_float2(x.x - y.y, x.y + y.x);
