@@ -364,7 +364,8 @@ __device__ __forceinline__ bool owner_heads(const OwnerCoef& c, const float* __r
         const bool go = __shfl_sync(kFull, (int)(has && more), lead) != 0;
         if (!__any_sync(kFull, go)) break;
         const int first = __shfl_sync(kFull, walk.first, lead);
-        const int edges = go ? __shfl_sync(kFull, walk.taken, lead) - first : (__shfl_sync(kFull, walk.taken, lead), 0);
+        const int taken = __shfl_sync(kFull, walk.taken, lead);   // by the whole warp: `go` differs between its groups
+        const int edges = go ? taken - first : 0;
         const int used = __shfl_sync(kFull, walk.used, lead);
         const bool wide = __shfl_sync(kFull, (int)walk.wide, lead) != 0;
         if (go)
