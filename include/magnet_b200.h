@@ -37,7 +37,8 @@ const char* mg_last_error(void);
 int mg_version(void);
 /* Stream used by this host thread's calls (a cudaStream_t; NULL = the legacy default stream). */
 int mg_set_stream(void* stream);
-/* Waits for all work of this host thread's stream. */
+/* Waits for all work of this host thread's stream. MG_ERR_TIMEOUT: an owner-mode run of this thread on device arrays
+ * gave up at one of its bounded waits (such a call returns before that is known), and its layout is not valid. */
 int mg_synchronize(void);
 /* Number of device kernels this library has launched in the process so far (a CUDA-graph replay counts each
  * kernel node). */

@@ -205,9 +205,6 @@ extern "C" int mg_set_stream(void* stream) {
     g_stream = static_cast<cudaStream_t>(stream);
     return MG_OK;
 }
-extern "C" int mg_synchronize(void) {
-    return guard([&] { MGB_CUDA(cudaStreamSynchronize(current_stream())); });
-}
 extern "C" uint64_t mg_launch_count(void) { return launch_count(); }
 
 // ============================================================================================== FFTConv2D
@@ -633,6 +630,13 @@ extern "C" int mg_optimize_layout(const mg_layout_args* a) {
             if (a->parallel == 1) owner_finish(*g_sgd_work, s);
             else MGB_CUDA(cudaStreamSynchronize(s));
         }
+    });
+}
+
+extern "C" int mg_synchronize(void) {
+    return guard([&] {
+        if (g_sgd_work) owner_finish(*g_sgd_work, current_stream());
+        else MGB_CUDA(cudaStreamSynchronize(current_stream()));
     });
 }
 

@@ -120,11 +120,24 @@ __device__ __forceinline__ void owner_step(const SgdDev& c, float* yu, const flo
         if (d < dim) yu[d] += step[d];
 }
 
+// What a thread whose work others wait for at a grid barrier tells them: one count per 256 units of work (a draw, an edge,
+// a copied value, a listing; at most a few microseconds each), so the count moves at least every millisecond or so.
+struct Beat {
+    unsigned* at;
+    unsigned done = 0;
+    __device__ __forceinline__ void tick() {
+        if ((++done & 255u) == 0u) atomicAdd(at, 1u);
+    }
+};
+struct NoBeat {   // of a launch in which nobody waits
+    __device__ __forceinline__ void tick() {}
+};
+
 // The edges of head node u in one epoch, from stream state `state`; returns the state after them. The row is read
 // from the snapshot and written back to Y (when u may move). `jitter` is set when a negative lands at distance 0.
-template <int D>
+template <int D, class B>
 __device__ uint64_t owner_node(const SgdDev& c, const OwnerDev& o, int64_t u, uint64_t state, float alpha,
-                               float mid_w, bool& jitter) {
+                               float mid_w, bool& jitter, B& beat) {
     constexpr int DM = D ? D : kMaxDim;
     const int dim = D ? D : c.dim;
     Rng r(0);
@@ -139,6 +152,7 @@ __device__ uint64_t owner_node(const SgdDev& c, const OwnerDev& o, int64_t u, ui
     for (int64_t w0 = o.row[u]; w0 < row1; w0 += 64) {
         // the sampled edges of a window of 64 as a bit mask, taken in edge order
         const int cnt = (int)(row1 - w0 < 64 ? row1 - w0 : 64);
+        beat.tick();
         uint64_t mask = 0;
         for (int t = 0; t < cnt; ++t)
             if (o.n_neg[w0 + t] != kNotSampled) mask |= 1ull << t;
@@ -146,6 +160,7 @@ __device__ uint64_t owner_node(const SgdDev& c, const OwnerDev& o, int64_t u, ui
             const int64_t i = w0 + (__ffsll((long long)mask) - 1);
             mask &= mask - 1;
             const int n_neg = o.n_neg[i];
+            beat.tick();
             const int32_t v = c.tail[i];
             const float* yv = o.Yr + (int64_t)v * dim;
             float d2 = 0.0f;
@@ -169,6 +184,7 @@ __device__ uint64_t owner_node(const SgdDev& c, const OwnerDev& o, int64_t u, ui
             // repulsion from the negatives, read from the snapshot
             for (int p = 0; p < n_neg; ++p) {
                 const int32_t k = (int32_t)r.below((uint32_t)c.n);
+                beat.tick();
                 if (k == u) continue;
                 const float* yk = o.Yr + (int64_t)k * dim;
                 float dd = 0.0f;
@@ -302,9 +318,11 @@ struct HeadWalk {
     int first, used;        // the round: its first edge in the list, its slots
     bool wide;              // the round is one edge of more negatives than the slots hold: drawn as it is computed
     uint64_t stream;
+    Beat beat;
 
     __device__ __forceinline__ void fill(const int32_t* __restrict__ rec, const int32_t* __restrict__ tails, EpochShared& sh) {
         const int cnt = (int)(row1 - w0 < kRowList ? row1 - w0 : kRowList);
+        beat.tick();
         have = 0; taken = 0;
         for (int t0 = 0; t0 < cnt; t0 += 8) {
             int nn[8], tt[8];
@@ -326,6 +344,7 @@ struct HeadWalk {
         while (taken < have) {
             const int2 e = sh.edge[taken][col];
             const int nn = e.x > 0 ? e.x : 0;
+            beat.tick();
             if (used + 1 + nn > kSlots) {
                 if (used > 0) break;
                 wide = true;
@@ -412,6 +431,7 @@ __device__ __forceinline__ bool owner_heads(const OwnerCoef& c, const float* __r
                 if (act && wide && gl == 0)
                     for (int t = 0; t < nn; ++t) {
                         xorshift(walk.stream);
+                        walk.beat.tick();
                         const int32_t k = below_state(walk.stream, n);
                         if (k != (int32_t)u) add_negative(c, yu, ld2(Yr, k), gu, jitter);
                     }
@@ -654,25 +674,32 @@ __global__ void __launch_bounds__(128) owner_node_kernel(SgdDev c, OwnerDev o, f
     const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (u >= c.n || o.row[u] == o.row[u + 1]) return;
     bool jitter = false;
-    owner_node<D>(c, o, u, o.state[o.row[u]], alpha, mid_w, jitter);
+    NoBeat none;
+    owner_node<D>(c, o, u, o.state[o.row[u]], alpha, mid_w, jitter, none);
     if (jitter) atomicExch(&o.dirty[chunk_of(o, u)], 1);
 }
 
 // the marked chunk k replayed serially from its seed; rows without edges never move
-template <int D>
+template <int D, class B>
 __device__ __noinline__ void owner_replay(const SgdDev& c, const OwnerDev& o, int k, int epoch, float alpha,
-                                          float mid_w) {
+                                          float mid_w, B beat) {
     // the heads of the chunk's edges (a marked chunk has at least one)
     const int64_t u0 = c.head[o.eown[k]], u1 = (int64_t)c.head[o.eown[k + 1] - 1] + 1;
     const int dim = c.dim;
-    for (int64_t j = u0 * dim; j < u1 * dim; ++j) c.Y[j] = o.Yr[j];
+    for (int64_t j = u0 * dim; j < u1 * dim; ++j) {
+        c.Y[j] = o.Yr[j];
+        beat.tick();
+    }
     if (c.optimizer == 1) {
         for (int64_t j = u0 * dim; j < u1 * dim; ++j) { c.adam_m[j] = o.snap_m[j]; c.adam_v[j] = o.snap_v[j]; }
         for (int64_t u = u0; u < u1; ++u) c.adam_t[u] = o.snap_t[u];
     }
     uint64_t state = Rng(stream_seed(c.seed, epoch, (uint64_t)k)).s;
     bool jitter = false;
-    for (int64_t u = u0; u < u1; ++u) state = owner_node<D>(c, o, u, state, alpha, mid_w, jitter);
+    for (int64_t u = u0; u < u1; ++u) {
+        beat.tick();
+        state = owner_node<D>(c, o, u, state, alpha, mid_w, jitter, beat);
+    }
 }
 
 template <int D>
@@ -681,7 +708,7 @@ __global__ void __launch_bounds__(32) owner_fallback_kernel(SgdDev c, OwnerDev o
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= o.n_chunks || !o.dirty[k]) return;
     o.dirty[k] = 0;
-    owner_replay<D>(c, o, k, epoch, alpha, mid_w);
+    owner_replay<D>(c, o, k, epoch, alpha, mid_w, NoBeat());
 }
 
 template <int D>
@@ -693,12 +720,16 @@ void owner_epoch_launch(const SgdDev& c, const OwnerDev& o, int epoch, float alp
 }
 
 // Grid barrier of a cooperative launch, in two halves: every block arrives on a counter that only grows, then waits for
-// all. The wait gives up after about a second (never reached while the launch's blocks run), sets *err and lets the
-// kernel end.
+// all. What it waits for has no bound of its own (a marked chunk is replayed by one thread, and a chunk may hold every
+// edge of the call; a row may draw any number of negatives), so the wait ends without the others only when kPolls polls
+// (one to three seconds) pass in which neither a block arrived nor a working thread's beat moved: it then sets *err
+// and lets the kernel end. While every block runs, the polls that see no beat stay far below that.
 struct GridBarrier {
     unsigned* count;
+    unsigned* beat;
     int* err;
     unsigned passed = 0;
+    static constexpr int kPolls = 4000000;
     __device__ __forceinline__ void arrive() {
         ++passed;
         __syncthreads();
@@ -711,10 +742,18 @@ struct GridBarrier {
         __shared__ int ok;
         if (threadIdx.x == 0) {
             const unsigned want = passed * gridDim.x;
+            unsigned arrived, seen_arrived = 0u, seen_beat = 0u;
             int tries = 0;
             int good = 1;
-            while (*reinterpret_cast<volatile unsigned*>(count) < want)
-                if (++tries > 4000000 || *reinterpret_cast<volatile int*>(err)) { atomicExch(err, 1); good = 0; break; }
+            while ((arrived = *reinterpret_cast<volatile unsigned*>(count)) < want) {
+                if (*reinterpret_cast<volatile int*>(err)) { good = 0; break; }
+                if (++tries < kPolls) continue;
+                const unsigned now = *reinterpret_cast<volatile unsigned*>(beat);
+                if (now == seen_beat && arrived == seen_arrived) { atomicExch(err, 1); good = 0; break; }
+                seen_beat = now;
+                seen_arrived = arrived;
+                tries = 0;
+            }
             __threadfence();
             ok = good;
         }
@@ -725,7 +764,8 @@ struct GridBarrier {
 
 // epoch `epoch`'s marked chunks, replayed by the grid's threads (its records at rec / state, layout Yr -> Yw)
 __device__ __noinline__ void owner_replay_marked(const SgdDev& call, const OwnerDev& own, int epoch, float alpha,
-                                                 const float* Yr, float* Yw, int32_t* rec, uint64_t* state) {
+                                                 const float* Yr, float* Yw, int32_t* rec, uint64_t* state,
+                                                 unsigned* beat) {
     SgdDev c = call;
     OwnerDev o = own;
     c.Y = Yw;
@@ -733,7 +773,7 @@ __device__ __noinline__ void owner_replay_marked(const SgdDev& call, const Owner
     for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < o.n_chunks; q += (int64_t)gridDim.x * blockDim.x)
         if (__ldcg(&o.dirty[q])) {
             o.dirty[q] = 0;
-            owner_replay<2>(c, o, (int)q, epoch, alpha, 0.0f);
+            owner_replay<2>(c, o, (int)q, epoch, alpha, 0.0f, Beat{beat});
         }
 }
 
@@ -748,7 +788,7 @@ __global__ void __launch_bounds__(kEpochThreads) owner_epochs_kernel(const __gri
                                                            int G, float* buf0, float* buf1,
                                                            const int32_t* __restrict__ heads,
                                                            const int* __restrict__ n_heads, int* __restrict__ any_dirty,
-                                                           unsigned* bar, int* err) {
+                                                           unsigned* bar, unsigned* beat, int* err) {
     extern __shared__ __align__(16) unsigned char epoch_smem[];
     EpochShared& sh = *reinterpret_cast<EpochShared*>(epoch_smem);
     const int gl = threadIdx.x & (G - 1);
@@ -760,13 +800,14 @@ __global__ void __launch_bounds__(kEpochThreads) owner_epochs_kernel(const __gri
     const int64_t n = c.n, n_fixed = c.n_fixed, E = c.n_edges;
     const int32_t* const tail = c.tail;
     const int64_t* const row = o.row;
-    GridBarrier barrier{bar, err};
+    GridBarrier barrier{bar, beat, err};
     // one head per group (every transform): its row bounds stay in registers, and the first round of an epoch is made
     // between the two halves of the barrier that ends the epoch before
     const bool single = work <= groups;
     int64_t u = -1, row0 = 0, row1 = 0;
     HeadWalk walk{};
     walk.col = threadIdx.x / G;
+    walk.beat.at = beat;
     bool more = false, has = false;
     auto head_at = [&](int64_t h) {
         u = heads ? (int64_t)heads[h] : h;
@@ -808,7 +849,7 @@ __global__ void __launch_bounds__(kEpochThreads) owner_epochs_kernel(const __gri
         if (single && has && gl == 0 && k + 1 < B) begin(k + 1);
         if (!barrier.wait()) return;
         if (__ldcg(&any_dirty[k])) {
-            owner_replay_marked(c, o, epoch, alpha, Yr, Yw, o.n_neg + (int64_t)k * E, o.state + (int64_t)k * E);
+            owner_replay_marked(c, o, epoch, alpha, Yr, Yw, o.n_neg + (int64_t)k * E, o.state + (int64_t)k * E, beat);
             barrier.arrive();
             if (!barrier.wait()) return;
         }
@@ -871,9 +912,14 @@ bool owner_heads_sorted(const int32_t* head_dev, int64_t n_edges, SgdWork& w, cu
 }
 
 void owner_finish(SgdWork& w, cudaStream_t s) {
+    if (!w.unasked) {
+        MGB_CUDA(cudaStreamSynchronize(s));
+        return;
+    }
     int gave_up = 0;
     MGB_CUDA(cudaMemcpyAsync(&gave_up, owner_flags(w, s) + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
     MGB_CUDA(cudaStreamSynchronize(s));
+    w.unasked = false;
     owner_check_timeout(gave_up, w, s);
 }
 
@@ -920,13 +966,13 @@ void owner_run(SgdDev& c, SgdWork& w, const int32_t* rev_indptr, const int32_t* 
     const bool pipelined = rows <= (int64_t)owner_resident_blocks() * kEpochThreads && dim == 2 && c.kernel == 0 && !c.node_b && !adam &&
                         (reinterpret_cast<uintptr_t>(Y) % sizeof(float2)) == 0;
     int32_t* heads = nullptr;
-    int* sync_words = nullptr;   // [0] barrier, [1] head count, [2 + k] epoch k of the batch marked a chunk
+    int* sync_words = nullptr;   // [0] barrier, [1] beat, [2] head count, [3 + k] epoch k of the batch marked a chunk
     if (pipelined) {
-        sync_words = static_cast<int*>(w.o_sync.ensure(sizeof(int) * (size_t)(2 + ahead)));
-        MGB_CUDA(cudaMemsetAsync(sync_words, 0, sizeof(int) * 2, s));
+        sync_words = static_cast<int*>(w.o_sync.ensure(sizeof(int) * (size_t)(3 + ahead)));
+        MGB_CUDA(cudaMemsetAsync(sync_words, 0, sizeof(int) * 3, s));
         if (c.n_fixed > 0) {
             heads = static_cast<int32_t*>(w.o_heads.ensure(sizeof(int32_t) * (size_t)E));
-            owner_heads_kernel<<<std::min(ceil_div(E, 256), 4 * kNumSMs), 256, 0, s>>>(c.head, E, heads, sync_words + 1);
+            owner_heads_kernel<<<std::min(ceil_div(E, 256), 4 * kNumSMs), 256, 0, s>>>(c.head, E, heads, sync_words + 2);
             MGB_LAUNCH_CHECK();
         }
     }
@@ -959,19 +1005,21 @@ void owner_run(SgdDev& c, SgdWork& w, const int32_t* rev_indptr, const int32_t* 
             SgdDev cc = c;
             if (run > 0) {
                 MGB_CUDA(cudaMemsetAsync(sync_words, 0, sizeof(int), s));
-                MGB_CUDA(cudaMemsetAsync(sync_words + 2, 0, sizeof(int) * (size_t)run, s));
+                MGB_CUDA(cudaMemsetAsync(sync_words + 3, 0, sizeof(int) * (size_t)run, s));
                 // lanes per head: 8 while the warps are at most one per scheduler
                 int G = 8;
                 while (G > 1 && rows * G > 4LL * kNumSMs * 32) G /= 2;
                 int blocks = (int)std::min<int64_t>(owner_resident_blocks(), std::max(1, ceil_div(rows * G, kEpochThreads)));
                 int b = b0 + k;
-                const int* n_heads = sync_words + 1;
-                int* any_dirty = sync_words + 2;
+                const int* n_heads = sync_words + 2;
+                int* any_dirty = sync_words + 3;
                 unsigned* bar = reinterpret_cast<unsigned*>(sync_words);
+                unsigned* beat = bar + 1;
                 int* err = owner_flags(w, s) + 1;
-                void* args[] = {&cc, &o, &sc, &b, &run, &G, &cur, &other, &heads, &n_heads, &any_dirty, &bar, &err};
+                void* args[] = {&cc, &o, &sc, &b, &run, &G, &cur, &other, &heads, &n_heads, &any_dirty, &bar, &beat, &err};
                 MGB_CUDA(cudaLaunchCooperativeKernel((const void*)owner_epochs_kernel, dim3(blocks), dim3(kEpochThreads), args, sizeof(EpochShared), s));
                 MGB_LAUNCH_CHECK();
+                w.unasked = true;
                 if (run & 1) std::swap(cur, other);
                 k += run;
                 continue;

@@ -45,6 +45,7 @@ struct SgdWork {
     // of the layout and the Adam state, the barrier and head count, the list of heads
     DevBuf o_row, o_own, o_neg, o_state, o_dirty, o_snap, o_snap_m, o_snap_v, o_snap_t, o_sync, o_heads;
     bool flags_ready = false;  // flag[1] (a grid barrier gave up) has been cleared once
+    bool unasked = false;      // a launch with grid barriers has run whose flag[1] has not been read since
     ~SgdWork() {
         if (totals) cudaFreeHost(totals);
         if (counted) cudaEventDestroy(counted);
@@ -66,8 +67,8 @@ void sgd_record(SgdDev& c, SgdWork& w, int stream_mode, int epoch, float alpha, 
 // s), and epochs [e0, e1); the reverse mid pairs are device arrays or NULL
 int owner_chunk_count(int64_t n_edges, int chunk_edges);
 bool owner_heads_sorted(const int32_t* head_dev, int64_t n_edges, SgdWork& w, cudaStream_t s);
-// waits for s and throws MG_ERR_TIMEOUT if a grid barrier of owner_run gave up (device-array calls learn of it from
-// the next call's owner_heads_sorted)
+// waits for s and throws MG_ERR_TIMEOUT if a grid barrier of owner_run gave up on it (calls on device arrays return before
+// that is known: mg_synchronize asks for them, and the next call's owner_heads_sorted)
 void owner_finish(SgdWork& w, cudaStream_t s);
 void owner_run(SgdDev& c, SgdWork& w, const int32_t* rev_indptr, const int32_t* rev_indices, int chunk_edges,
                int e0, int e1, float alpha0, float alpha1, float mid_w0, float mid_w1, cudaStream_t s);

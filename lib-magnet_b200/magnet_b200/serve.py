@@ -337,6 +337,8 @@ class FittedLayout:
                               self.a, self.b, self.rep_a, self.rep_b, 5.0, 0, 1.0, 2.0, 4, 0.25, 0, 0, self.n,
                               z2, z2, z, 0.9, 0.999, z, np.zeros((0, 1), np.int32), z, z, 0.0, 0, zf, sd, -1,
                               self.parallel, None, None, 0, owner_chunk_edges=self.chunk_edges)
+            if _lib().mg_synchronize() != 0:   # an owner run that gave up: its positions are not valid
+                raise RuntimeError(_lib().mg_last_error().decode())
             out = Y_all[self.n:].cpu().numpy()
         return out
 
