@@ -228,7 +228,7 @@ extern "C" int mg_fftconv_create(int M, int n_interp, mg_fftconv** out) {
         h->gdesc.ensure(sizeof(GridDesc));
         cudaStream_t s = current_stream();
         MGB_CUDA(cudaMemsetAsync(h->gdesc.p, 0, sizeof(GridDesc), s));
-        rep_set_grid_host(h->gdesc.as<GridDesc>(), 0.f, 0.f, 1.f, 1, n_interp, M, s);
+        rep_set_grid(h->gdesc.as<GridDesc>(), nullptr, 0, 0.f, 0.f, 1.f, 1, n_interp, M, h->rb.use3, s);
         rep_twiddles(h->gdesc.as<GridDesc>(), h->rb, s, true);
         MGB_CUDA(cudaStreamSynchronize(s));
         *out = h.release();
@@ -262,8 +262,8 @@ extern "C" int mg_fftconv_compute(mg_fftconv* h, const float* Y, int64_t n, floa
         require(sumQ != nullptr && (F != nullptr || n == 0), "sumQ and F must not be NULL");
         cudaStream_t s = current_stream();
         GridDesc* g = h->gdesc.as<GridDesc>();
-        rep_set_grid_host(g, xmin, ymin, width, n_boxes, h->ni, h->M, s);
         const float2* Yd = reinterpret_cast<const float2*>(in_dev(Y, 2 * n, 2, s));
+        rep_set_grid(g, Yd, n, xmin, ymin, width, n_boxes, h->ni, h->M, h->rb.use3, s);
         float2* Fd = reinterpret_cast<float2*>(out_dev(F, 2 * n, 3));
         if (n > 0) rep_spread(Yd, n, g, h->rb, s);
         rep_convolve(g, h->rb, n, s);

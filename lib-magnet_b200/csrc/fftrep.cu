@@ -91,6 +91,7 @@ __global__ void __launch_bounds__(256) spread_kernel(const float2* __restrict__ 
                                                      const GridDesc* __restrict__ gd, float4* __restrict__ W,
                                                      int pitch) {
     const float xmin = gd->xmin, ymin = gd->ymin, width = gd->width, inv_w = gd->inv_width;
+    const float2 up = gd->up;
     const int nb = gd->n_boxes;
     const int lane = threadIdx.x & 31;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -103,6 +104,7 @@ __global__ void __launch_bounds__(256) spread_kernel(const float2* __restrict__ 
         float wx[NI], wy[NI];
         locate<NI>(x, y, xmin, ymin, width, inv_w, nb, bx, by, wx, wy);
         const int key = act ? bx * nb + by : -1;
+        x *= up.x; y *= up.y;
         const unsigned peers = __match_any_sync(0xffffffffu, key);
         if (peers == 0xffffffffu && key >= 0) {
             // whole warp in one box: reduce per node, lane q issues node q
@@ -428,7 +430,35 @@ __global__ void transpose_spectra_kernel(const float* __restrict__ K, float* __r
     }
 }
 
-__global__ void set_grid_kernel(GridDesc* gd, float xmin, float ymin, float width, int n_boxes, int ni, int M) {
+// the caller's grid, and the scale of the charges from the points' largest coordinates (the last block writes both)
+__global__ void __launch_bounds__(256) set_grid_kernel(GridDesc* gd, const float2* __restrict__ Y, int64_t n, float xmin,
+                                                       float ymin, float width, int n_boxes, int ni, int M, bool in_place) {
+    __shared__ unsigned peak[2];
+    __shared__ int is_last;
+    if (threadIdx.x < 2) peak[threadIdx.x] = 0u;
+    float ax = 0.f, ay = 0.f;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const float2 p = Y[i];
+        ax = fmaxf(ax, fabsf(p.x)); ay = fmaxf(ay, fabsf(p.y));
+    }
+    __syncthreads();
+    const unsigned mx = __reduce_max_sync(0xffffffffu, __float_as_uint(ax));
+    const unsigned my = __reduce_max_sync(0xffffffffu, __float_as_uint(ay));
+    if ((threadIdx.x & 31) == 0) { atomicMax(&peak[0], mx); atomicMax(&peak[1], my); }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        atomicMax(&gd->peak[0], peak[0]);
+        atomicMax(&gd->peak[1], peak[1]);
+        __threadfence();
+        is_last = atomicAdd(&gd->counter2, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!is_last || threadIdx.x != 0) return;
+    __threadfence();
+    ax = __uint_as_float(__ldcg(&gd->peak[0])); ay = __uint_as_float(__ldcg(&gd->peak[1]));
+    gd->peak[0] = 0u; gd->peak[1] = 0u; gd->counter2 = 0u;
+    if (in_place) set_field_scale(gd, ax, ay);
+    else gd->up = gd->down = make_float2(1.f, 1.f);
     gd->xmin = xmin; gd->ymin = ymin; gd->width = width; gd->inv_width = 1.f / width;
     gd->n_boxes = n_boxes; gd->N = n_boxes * ni; gd->M = M; gd->Mh = M / 2 + 1;
 }
@@ -460,9 +490,10 @@ void gather_t(const float2* Y, int64_t n, GridDesc* g, RepBuffers& b, float2* F,
 
 }  // namespace
 
-void rep_set_grid_host(GridDesc* g_dev, float xmin, float ymin, float width, int n_boxes, int ni, int M,
-                       cudaStream_t s) {
-    set_grid_kernel<<<1, 1, 0, s>>>(g_dev, xmin, ymin, width, n_boxes, ni, M);
+void rep_set_grid(GridDesc* g_dev, const float2* Y, int64_t n, float xmin, float ymin, float width, int n_boxes, int ni,
+                  int M, bool in_place, cudaStream_t s) {
+    const int blocks = in_place ? (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 4 * kNumSMs)) : 1;
+    set_grid_kernel<<<blocks, 256, 0, s>>>(g_dev, Y, in_place ? n : 0, xmin, ymin, width, n_boxes, ni, M, in_place);
     MGB_LAUNCH_CHECK();
 }
 

@@ -1,14 +1,14 @@
 // The FFT repulsion's three transforms on the in-place engine (fft3.cuh): forward rows, columns with the kernel
 // products, inverse rows (src/fftconv.cpp:124-199), and the FP64 Z of :226-229.
 //
-// The three real charge fields run as two transforms. x W and y W are packed as one complex field x W + i y W: its
-// column products with the real kernel spectrum give phi_2 + i phi_3, so nothing is ever separated and its spectrum
-// stays in the order the stages leave (row position p of the transposed buffer holds frequency freq_of_pos(p)). The
+// The three real charge fields run as two transforms. x W and y W are packed as one complex field 2^j x W +
+// i 2^k y W (set_field_scale): its column products with the real kernel spectrum give 2^j phi_2 + i 2^k phi_3, so nothing is ever
+// separated and its spectrum stays in the order the stages leave (row position p of the transposed buffer holds frequency freq_of_pos(p)). The
 // charge field W needs its own spectrum for Z; two of its rows share a transform, separated into half spectra after
 // the forward rows and rebuilt before the inverse ones.
 //
-// Work items: rows by pairs (x W + i y W) or fours (W), columns by position (x W + i y W) or frequency (W), one per
-// block at a time. The items of all layouts of a launch are one list, dealt over the resident blocks.
+// Work items: rows by pairs (the complex field) or fours (W), columns by position (the complex field) or frequency (W),
+// one per block at a time. The items of all layouts of a launch are one list, dealt over the resident blocks.
 //
 //   columns: the first forward stage reads the live rows (g < N) from global memory, the last inverse stage writes the
 //   live rows, so a column costs 2 (S - 1) shared-memory passes per transform and no reordering pass.
@@ -328,16 +328,16 @@ struct ChargeStore {
         if (gb < N) phi[(size_t)gb * pitch + n] = v.y * scale;
     }
 };
-// potentials 2 (Re) and 3 (Im) of row g0 + t
+// potentials 2 (Re, times 2^j) and 3 (Im, times 2^k) of row g0 + t
 struct FieldStore {
     float* phi2;
     float* phi3;
     int pitch, g0;
-    float scale;
+    float scale2, scale3;   // 2^-j / M^2, 2^-k / M^2
     __device__ __forceinline__ void operator()(int t, int n, float2 v) const {
         const size_t at = (size_t)(g0 + t) * pitch + n;
-        phi2[at] = v.x * scale;
-        phi3[at] = v.y * scale;
+        phi2[at] = v.x * scale2;
+        phi3[at] = v.y * scale3;
     }
 };
 
@@ -473,7 +473,7 @@ __global__ void __launch_bounds__(kRowThreads, kRowBlocks) row_inv3_kernel(const
                                     ChargeStore{L.phi + plane, L.Nmax, g0, N, scale}, N, tw);
         } else {
             MGB_FFT3_RADIX_DISPATCH(p.st[0].R, fft3::dit_last, p, 0, p.Mp, nbuf,
-                                    FieldStore{L.phi + 2 * plane, L.phi + 3 * plane, L.Nmax, g0, scale}, N, tw);
+                                    FieldStore{L.phi + 2 * plane, L.phi + 3 * plane, L.Nmax, g0, scale * L.g->down.x, scale * L.g->down.y}, N, tw);
         }
         __syncthreads();
     }

@@ -132,7 +132,7 @@ void fftconv_compute_noalloc(const float* K1h, const float* K2h, int M, int n_in
     const int N = n_boxes * n_interp;
     MGB_CUDA(cudaMemsetAsync(g, 0, sizeof(GridDesc), s));
     MGB_CUDA(cudaMemsetAsync(base + kWOff, 0, (size_t)N * kNoallocMaxM * sizeof(float4), s));
-    rep_set_grid_host(g, xmin, ymin, width, n_boxes, n_interp, M, s);
+    rep_set_grid(g, nullptr, 0, xmin, ymin, width, n_boxes, n_interp, M, false, s);
     rep_twiddles(g, v.rb, s, true);
     rep_set_spectra_from_host_layout(v.rb, K1h, K2h, M, s);
     const float2* Yd = reinterpret_cast<const float2*>(Y);

@@ -218,6 +218,7 @@ __device__ void choose_grid(GridDesc* g, BBox b, const TsneSched& s, const int* 
     nb = min(s.max_boxes, (nb + 3) / 4 * 4);
     const double width = ((double)nb * s.box_width >= span) ? s.box_width : fmax(span / (double)nb, 1e-12);
     g->xmin = (float)lo0; g->ymin = (float)lo1;
+    set_field_scale(g, fmaxf(fabsf(b.x0), fabsf(b.x1)), fmaxf(fabsf(b.y0), fabsf(b.y1)));
     g->width = (float)width; g->inv_width = 1.f / g->width;
     g->n_boxes = nb; g->N = nb * s.ni;
     const int M = fft_len[2 * g->N];
@@ -278,7 +279,7 @@ __global__ void __launch_bounds__(kThreads) loop_start_kernel(const __grid_const
     if (L.g->tw_dirty) make_twiddles(L.tw, L.g->M);
 }
 
-// The spread of the charges (1, x, y) of a layout's points, recentred on the way (Ycur = Ynext - mean): one thread per
+// The spread of the charges (1, 2^j x, 2^k y) of a layout's points, recentred on the way (Ycur = Ynext - mean): one thread per
 // point, nodes accumulated with vector float atomics. Warps whose 32 points share one box (the dense case:
 // early-exaggeration layouts put everything in a few boxes) first reduce the node values with shuffles, so one atomic
 // per node replaces 32. Layout blockIdx.y.
@@ -287,6 +288,7 @@ __global__ void __launch_bounds__(256) loop_spread_kernel(const __grid_constant_
     const LoopDesc& L = MANY ? args.many[blockIdx.y] : args.one;
     const GridDesc* gd = L.g;
     const float xmin = gd->xmin, ymin = gd->ymin, width = gd->width, inv_w = gd->inv_width;
+    const float2 up = gd->up;
     const int nb = gd->n_boxes;
     const bool rc = gd->recentre != 0;
     const float mx = gd->mean[0], my = gd->mean[1];
@@ -308,6 +310,7 @@ __global__ void __launch_bounds__(256) loop_spread_kernel(const __grid_constant_
         float wx[NI], wy[NI];
         locate<NI>(x, y, xmin, ymin, width, inv_w, nb, bx, by, wx, wy);
         const int key = act ? bx * nb + by : -1;
+        x *= up.x; y *= up.y;
         const int key0 = __shfl_sync(0xffffffffu, key, 0);
         const bool one_box = __all_sync(0xffffffffu, act && key == key0) != 0;
         if (one_box) {
