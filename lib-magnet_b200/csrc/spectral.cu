@@ -5,10 +5,13 @@
 // Kernels:
 //  * step_kernel, one degree of the filter in one launch: the product with the lazy normalised adjacency (a group of
 //    lanes per row, one per column, each summing the row's entries in order, as src/spectral.cpp:34-48), the deflation
-//    of the trivial eigenvector per connected component, and the three-term recurrence. The trivial eigenvector t is an
-//    eigenvector of M for 1, so the projection of M Y on it is that of Y, which the step before has summed while it
-//    wrote Y (per-component sums by block reductions and FP64 atomics): no pass between the product and the recurrence.
-//    The block is kept twice, as it is and with its rows scaled by D^-1/2 (what the next product gathers);
+//    of the trivial eigenvector t per component, and the three-term recurrence. The projection of M Y on t is that of Y on
+//    u = M^T t, which the step before has summed while it wrote Y (per-component sums by block reductions and FP64
+//    atomics): no pass between the product and the recurrence. On the graph's own degrees u is t but for inv_sqrt_deg's
+//    rounding, and is held as u / t - 1 in single precision (to 1e-11 of t), read where it is used (read with the row's
+//    other values the step took 45 us instead of 37). Where it is not (other scale factors, a directed graph), or an
+//    edge joins two components, the steps take the product and the rest in two launches (finish_kernel). The block is
+//    kept twice, as it is and with its rows scaled by D^-1/2 (what the next product gathers);
 //  * the p x p products X^T X and X^T Z summed over the rows inside the kernels that write X or Z, the blocks' partial
 //    sums added in a fixed order by the last block;
 //  * two passes of Cholesky orthonormalisation (X <- X R^-1 with X^T X = R^T R, which is Gram-Schmidt of the columns in
@@ -16,7 +19,7 @@
 //    for it goes column by column;
 //  * the rotation by the Ritz vectors with the residuals. The p x p factorisations and eigenproblem run on the host.
 // Bound by the gathers of the products (one 8 p byte row per entry from L2) and their index reads. At 200k rows of 25
-// entries, p = 4: 36 us per degree (140 G gathered rows/s) against 65 as five passes (product 48, component sums 4.6, deflation
+// entries, p = 4: 37 us per degree (136 G gathered rows/s) against 65 as five passes (product 48, component sums 4.6, deflation
 // 6.4, recurrence 4.8), and 4 host round trips per outer iteration against 33.
 #include "spectral.cuh"
 #include <algorithm>
@@ -115,13 +118,14 @@ __device__ __forceinline__ void sum_partials(const double* __restrict__ part, un
 // One step Yout = (Z - c Yin) s - ss X with Z = M Yin deflated, M = (I + D^-1/2 A D^-1/2) / 2. Vin = D^-1/2 Yin is what
 // the product gathers, Vout the same of Yout; X may be Yout (each entry is read before it is written). proj_in holds the
 // per-component sums of t Yin, proj_out (zero before) receives those of t Yout, proj_next is set to zero for the step
-// after. GRAM: part / counter / gram receive the p x p product Yin^T Yout.
+// after. GRAM: part / counter / gram receive the p x p product Yin^T Yout. du: the sums are those of t (1 + du) Yout, as
+// the next product wants them (zeros: of t Yout).
 template <int P, bool GRAM>
 __global__ void __launch_bounds__(kSpecThreads) step_kernel(
     const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices, const float* __restrict__ data,
     const float* __restrict__ sd, const int32_t* __restrict__ comp, const double* __restrict__ tnorm, int64_t n,
-    int64_t n_proj, const double* __restrict__ Yin, const double* __restrict__ Vin, const double* X, double* Yout,
-    double* __restrict__ Vout, double c, double s, double ss, const double* __restrict__ proj_in,
+    const float* __restrict__ du, int64_t n_proj, const double* __restrict__ Yin, const double* __restrict__ Vin,
+    const double* X, double* Yout, double* __restrict__ Vout, double c, double s, double ss, const double* __restrict__ proj_in,
     double* __restrict__ proj_out, double* __restrict__ proj_next, double* __restrict__ part,
     unsigned* __restrict__ counter, double* __restrict__ gram) {
     constexpr int G = kLanes<P>;
@@ -191,7 +195,7 @@ __global__ void __launch_bounds__(kSpecThreads) step_kernel(
             if (ss != 0.0) out -= ss * xo;
             Yout[i * P + k] = out;
             Vout[i * P + k] = (double)sdi * out;
-            cs.add(t * out, cc, proj_out, P, k);
+            cs.add((t + t * (double)du[i]) * out, cc, proj_out, P, k);
         }
         if constexpr (GRAM) {
 #pragma unroll
@@ -222,17 +226,125 @@ __global__ void __launch_bounds__(kSpecThreads) trivial_norm_kernel(const float*
     flush_component<1, 1>(cs, tnorm, 0, red);
 }
 
+// u = M^T t: u_j = (t_j + sd_j sum_i a_ij sd_i t_i) / 2, by one warp per row; `u` holds t / 2 before. *open: an edge joins
+// two components, for which the projections have no such weights.
+__global__ void __launch_bounds__(kSpecThreads) half_trivial_kernel(const float* __restrict__ sd, int64_t n, double* __restrict__ u) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        u[i] = 0.5 * trivial_of(sd[i]);
+}
+__global__ void __launch_bounds__(kSpecThreads) adjoint_kernel(const int32_t* __restrict__ indptr, const int32_t* __restrict__ indices,
+                                                               const float* __restrict__ data, const float* __restrict__ sd,
+                                                               const int32_t* __restrict__ comp, int64_t n,
+                                                               int n_comp, double* __restrict__ u, int* __restrict__ open) {
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    bool crosses = false;
+    for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
+        const double st = (double)sd[i] * trivial_of(sd[i]);
+        if (st == 0.0) continue;
+        const int c = comp[i];
+        const int32_t e1 = indptr[i + 1];
+        for (int32_t e = indptr[i] + lane; e < e1; e += 32) {
+            const int32_t j = indices[e];
+            const double x = 0.5 * (double)sd[j] * ((double)data[e] * st);
+            if (x == 0.0) continue;
+            if (n_comp == 1 || comp[j] == c) atomicAdd(&u[j], x);
+            else crosses = true;
+        }
+    }
+    if (crosses) *open = 1;
+}
+// u / t - 1 as it is held, *open where that is no small number
+__global__ void __launch_bounds__(kSpecThreads) ratio_kernel(const float* __restrict__ sd, const double* __restrict__ u, int64_t n,
+                                                             float* __restrict__ du, int* __restrict__ open) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const double t = trivial_of(sd[i]);
+        const double r = t > 0.0 ? u[i] / t - 1.0 : (u[i] == 0.0 ? 0.0 : INFINITY);
+        du[i] = (float)r;
+        if (!(fabs(r) < 1e-4)) *open = 1;
+    }
+}
+
 template <int P>
 struct Coef {
     double v[P * P];
 };
+
+// the sums of P columns, one thread per row
+template <int P>
+__device__ __forceinline__ void flush_rows(ComponentSum (&cs)[P], double* __restrict__ proj, double (*red)[1]) {
+    __shared__ int any;
+    if (threadIdx.x == 0) any = -1;
+    __syncthreads();
+    if (cs[0].comp >= 0) any = cs[0].comp;
+    __syncthreads();
+    const int c = any;
+    const bool one = __syncthreads_and(cs[0].comp < 0 || cs[0].comp == c) != 0;
+#pragma unroll
+    for (int k = 0; k < P; ++k) {
+        if (one) {
+            const double t = column_block_sum<1>(cs[k].comp >= 0 ? cs[k].sum : 0.0, red);
+            if (threadIdx.x == 0 && c >= 0) atomicAdd(&proj[(int64_t)c * P + k], t);
+        } else if (cs[k].comp >= 0) {
+            atomicAdd(&proj[(int64_t)cs[k].comp * P + k], cs[k].sum);
+        }
+    }
+}
+
+// The rest of a step whose product Z = M Yin stands by itself: Yout = (Z deflated - c Yin) s - ss X, with proj_in the
+// per-component sums of t Z; the other outputs as step_kernel's (proj_out those of t Yout).
+template <int P, bool GRAM>
+__global__ void __launch_bounds__(kSpecThreads) finish_kernel(const float* __restrict__ sd, const int32_t* __restrict__ comp,
+                                                              const double* __restrict__ tnorm, int64_t n,
+                                                              const double* __restrict__ Z, const double* __restrict__ Yin,
+                                                              const double* X, double* Yout, double* __restrict__ Vout,
+                                                              double c, double s, double ss, const double* __restrict__ proj_in,
+                                                              double* __restrict__ proj_out, double* __restrict__ part,
+                                                              unsigned* __restrict__ counter, double* __restrict__ gram) {
+    __shared__ double red[kSpecThreads / 32][1];
+    double acc[GRAM ? P * P : 1];
+#pragma unroll
+    for (int q = 0; q < (GRAM ? P * P : 1); ++q) acc[q] = 0.0;
+    ComponentSum cs[P];
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const double sdi = (double)sd[i], t = trivial_of(sd[i]);
+        const int cc = comp[i];
+        const double tn = tnorm[cc];
+        double y[P], out[P];
+#pragma unroll
+        for (int k = 0; k < P; ++k) {
+            y[k] = Yin[i * P + k];
+            const double z = Z[i * P + k] - t * (tn > 0.0 ? proj_in[(int64_t)cc * P + k] / tn : 0.0);
+            out[k] = (z - c * y[k]) * s;
+            if (ss != 0.0) out[k] -= ss * X[i * P + k];
+            Yout[i * P + k] = out[k];
+            Vout[i * P + k] = sdi * out[k];
+            cs[k].add(t * out[k], cc, proj_out, P, k);
+        }
+        if constexpr (GRAM) {
+#pragma unroll
+            for (int a = 0; a < P; ++a)
+#pragma unroll
+                for (int q = 0; q < P; ++q) acc[a * P + q] += y[a] * out[q];
+        }
+    }
+    flush_rows<P>(cs, proj_out, red);
+    if constexpr (GRAM) {
+#pragma unroll
+        for (int q = 0; q < P * P; ++q) {
+            const double t = column_block_sum<1>(acc[q], red);
+            if (threadIdx.x == 0) part[(size_t)blockIdx.x * P * P + q] = t;
+        }
+        sum_partials<P * P>(part, counter, gram);
+    }
+}
 
 // The rows of a P-column block, one thread per row (compile-time switches):
 //  WIDEN    X from the caller's float block
 //  DEFLATE  X -= t proj_in / tnorm
 //  APPLY    X <- X T (column c = sum_k X_k T[k][c])
 //  GRAM     gram = X^T X of what was written
-//  SUMS     V = D^-1/2 X and proj_out = per-component sums of t X
+//  SUMS     V = D^-1/2 X and proj_out = per-component sums of t (1 + du) X
 //  RESID    resid[c] = sum of ((Z T)_ic - theta_c X_ic)^2
 constexpr int kWiden = 1, kDeflate = 2, kApply = 4, kGram = 8, kSums = 16, kResid = 32;
 
@@ -240,7 +352,7 @@ template <int P, int USE>
 __global__ void __launch_bounds__(kSpecThreads) rows_kernel(const float* __restrict__ in, double* __restrict__ X,
                                                             const double* __restrict__ Z, int64_t n, Coef<P> T, Coef<P> theta,
                                                             const float* __restrict__ sd, const int32_t* __restrict__ comp,
-                                                            const double* __restrict__ tnorm,
+                                                            const double* __restrict__ tnorm, const float* __restrict__ du,
                                                             const double* __restrict__ proj_in, double* __restrict__ V,
                                                             double* __restrict__ proj_out, double* __restrict__ part,
                                                             unsigned* __restrict__ counter, double* __restrict__ out) {
@@ -296,10 +408,11 @@ __global__ void __launch_bounds__(kSpecThreads) rows_kernel(const float* __restr
 #pragma unroll
         for (int k = 0; k < P; ++k) X[i * P + k] = x[k];
         if constexpr ((USE & kSums) != 0) {
+            const double ws = t + t * (double)du[i];
 #pragma unroll
             for (int k = 0; k < P; ++k) {
                 if (V) V[i * P + k] = (double)sdi * x[k];
-                cs[k].add(t * x[k], c, proj_out, P, k);
+                cs[k].add(ws * x[k], c, proj_out, P, k);
             }
         }
         if constexpr ((USE & kGram) != 0) {
@@ -309,24 +422,7 @@ __global__ void __launch_bounds__(kSpecThreads) rows_kernel(const float* __restr
                 for (int q = 0; q < P; ++q) acc[r * P + q] += x[r] * x[q];
         }
     }
-    if constexpr ((USE & kSums) != 0) {
-        __shared__ int any;
-        if (threadIdx.x == 0) any = -1;
-        __syncthreads();
-        if (cs[0].comp >= 0) any = cs[0].comp;
-        __syncthreads();
-        const int c = any;
-        const bool one = __syncthreads_and(cs[0].comp < 0 || cs[0].comp == c) != 0;
-#pragma unroll
-        for (int k = 0; k < P; ++k) {
-            if (one) {
-                const double t = column_block_sum<1>(cs[k].comp >= 0 ? cs[k].sum : 0.0, red);
-                if (threadIdx.x == 0 && c >= 0) atomicAdd(&proj_out[(int64_t)c * P + k], t);
-            } else if (cs[k].comp >= 0) {
-                atomicAdd(&proj_out[(int64_t)cs[k].comp * P + k], cs[k].sum);
-            }
-        }
-    }
+    if constexpr ((USE & kSums) != 0) flush_rows<P>(cs, proj_out, red);
     if constexpr ((USE & (kGram | kResid)) != 0) {
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
@@ -372,6 +468,8 @@ struct Solver {
     int64_t n; int64_t n_proj; int blocks; int sblocks; cudaStream_t s;
     double* proj[3]; int at = 0;          // per-component sums of t X: proj[at] those of the current block
     const double* tnorm; double* part; unsigned* counter; double* sums; double* host;
+    const float* du; int open = 0;        // u / t - 1, then n zeros; u is no such thing (read with the first sums)
+    const double* no_norm; double* Z;     // zeros in the place of tnorm; the product of a step in two launches
 
     double* now() { return proj[at]; }
     double* next() { return proj[(at + 1) % 3]; }
@@ -383,20 +481,40 @@ struct Solver {
         MGB_CUDA(cudaStreamSynchronize(s));
         return host;
     }
+    // the p x p sums, with the open flag behind them
+    const double* read_flagged() {
+        const double* h = read(P * P + 1);
+        open = reinterpret_cast<const int*>(h + P * P)[1];
+        return h;
+    }
     template <int USE>
     void rows(double* X, const double* Z, const Coef<P>& T, const Coef<P>& theta, double* V, const float* in = nullptr) {
+        const float* w = in ? du + n : du;   // the caller's block is deflated next, the others multiplied
         if (USE & kSums) MGB_CUDA(cudaMemsetAsync(next(), 0, sizeof(double) * (size_t)n_proj, s));
-        rows_kernel<P, USE><<<blocks, kSpecThreads, 0, s>>>(in, X, Z, n, T, theta, sd, comp, tnorm, now(), V, next(), part,
+        rows_kernel<P, USE><<<blocks, kSpecThreads, 0, s>>>(in, X, Z, n, T, theta, sd, comp, tnorm, w, now(), V, next(), part,
                                                            counter, sums);
         MGB_LAUNCH_CHECK();
         if (USE & kSums) at = (at + 1) % 3;
     }
-    // Yout = ((M Yin deflated) - c Yin) s - ss X; proj moves on (the next target was zeroed by the step before, or here)
+    // Yout = ((M Yin deflated) - c Yin) s - ss X; proj moves on (the next target was zeroed by the step before, or here);
+    // last: Yout is deflated next, not multiplied
     template <bool GRAM>
     void step(const double* Yin, const double* Vin, const double* X, double* Yout, double* Vout, double c, double sc,
-              double ss, bool clear) {
+              double ss, bool clear, bool last) {
+        if (open) {
+            MGB_CUDA(cudaMemsetAsync(next(), 0, sizeof(double) * (size_t)n_proj, s));
+            step_kernel<P, false><<<sblocks, kSpecThreads, 0, s>>>(indptr, indices, data, sd, comp, no_norm, n, du + n, n_proj, Yin, Vin,
+                                                                  nullptr, Z, Vout, 0.0, 1.0, 0.0, now(), next(), after(), part,
+                                                                  counter, sums);
+            MGB_LAUNCH_CHECK();
+            finish_kernel<P, GRAM><<<blocks, kSpecThreads, 0, s>>>(sd, comp, tnorm, n, Z, Yin, X, Yout, Vout, c, sc, ss, next(),
+                                                                   after(), part, counter, sums);
+            MGB_LAUNCH_CHECK();
+            at = (at + 2) % 3;
+            return;
+        }
         if (clear) MGB_CUDA(cudaMemsetAsync(next(), 0, sizeof(double) * (size_t)n_proj, s));
-        step_kernel<P, GRAM><<<sblocks, kSpecThreads, 0, s>>>(indptr, indices, data, sd, comp, tnorm, n, n_proj, Yin, Vin, X,
+        step_kernel<P, GRAM><<<sblocks, kSpecThreads, 0, s>>>(indptr, indices, data, sd, comp, tnorm, n, last ? du + n : du, n_proj, Yin, Vin, X,
                                                              Yout, Vout, c, sc, ss, now(), next(), after(), part, counter, sums);
         MGB_LAUNCH_CHECK();
         at = (at + 1) % 3;
@@ -437,7 +555,7 @@ struct Solver {
     void orthonormalize(double* X, double* V) {
         rows<kDeflate | kGram>(X, nullptr, Coef<P>{}, Coef<P>{}, nullptr);
         Coef<P> T;
-        if (inverse_factor(read(P * P), T)) {
+        if (inverse_factor(read_flagged(), T)) {
             rows<kApply | kGram>(X, nullptr, T, Coef<P>{}, nullptr);
             if (inverse_factor(read(P * P), T)) {
                 rows<kApply | kSums>(X, nullptr, T, Coef<P>{}, V);
@@ -471,7 +589,7 @@ struct Solver {
     // rotated by V; returns the largest residual norm |Z_c - theta_c X_c| over the wanted columns. Vx: D^-1/2 X in and
     // out, Vz scratch.
     double rayleigh_ritz(double* X, double* Vx, double* Z, double* Vz, int n_wanted, std::vector<double>& theta) {
-        step<true>(X, Vx, nullptr, Z, Vz, 0.0, 1.0, 0.0, true);
+        step<true>(X, Vx, nullptr, Z, Vz, 0.0, 1.0, 0.0, true, true);
         const double* h = read(P * P);
         std::vector<double> H(h, h + P * P);
         for (int a = 0; a < P; ++a)
@@ -496,7 +614,8 @@ struct Solver {
         double* Vx = static_cast<double*>(w.Z.ensure(bytes));
         double* Vy = static_cast<double*>(w.Ynew.ensure(bytes));
         rows<kWiden | kSums>(X, nullptr, Coef<P>{}, Coef<P>{}, nullptr, Xout);
-        orthonormalize(X, Vx);
+        orthonormalize(X, Vx);   // (waits for the stream)
+        if (open) Z = static_cast<double*>(w.M.ensure(bytes));
         std::vector<double> theta;
         double res = rayleigh_ritz(X, Vx, Y, Vy, n_wanted, theta);
         double prev_sum = -1.0;
@@ -518,10 +637,10 @@ struct Solver {
             const double e = 0.5 * alpha, cc = 0.5 * alpha;
             const double sigma1 = e / (a0 - cc);
             double sigma = sigma1;
-            step<false>(X, Vx, nullptr, Y, Vy, cc, sigma1 / e, 0.0, true);
+            step<false>(X, Vx, nullptr, Y, Vy, cc, sigma1 / e, 0.0, true, false);
             for (int k = 2; k <= degree; ++k) {
                 const double sigma_new = 1.0 / (2.0 / sigma1 - sigma);
-                step<false>(Y, Vy, X, X, Vx, cc, 2.0 * sigma_new / e, sigma * sigma_new, false);
+                step<false>(Y, Vy, X, X, Vx, cc, 2.0 * sigma_new / e, sigma * sigma_new, false, k == degree);
                 std::swap(X, Y);
                 std::swap(Vx, Vy);
                 sigma = sigma_new;
@@ -549,19 +668,31 @@ void run_solver(const int32_t* indptr, const int32_t* indices, const float* data
                                                              (int64_t)kStepBlocks * kNumSMs));
     double* proj = static_cast<double*>(w.proj.ensure(sizeof(double) * 3 * (size_t)sv.n_proj));
     for (int q = 0; q < 3; ++q) sv.proj[q] = proj + q * sv.n_proj;
-    double* tn = static_cast<double*>(w.tnorm.ensure(sizeof(double) * (size_t)n_comp));
+    double* tn = static_cast<double*>(w.tnorm.ensure(2 * sizeof(double) * (size_t)n_comp));
+    sv.no_norm = tn + n_comp;
     // the block partials, the sums and the last-block counter
     const size_t parts = (size_t)std::max(sv.blocks, sv.sblocks) * P * P;
     sv.part = static_cast<double*>(w.part.ensure(sizeof(double) * (parts + P * P + 1)));
     sv.sums = sv.part + parts;
-    sv.counter = reinterpret_cast<unsigned*>(sv.sums + P * P);
-    double host[P * P];
+    sv.counter = reinterpret_cast<unsigned*>(sv.sums + P * P);   // and the open flag
+    int* open = reinterpret_cast<int*>(sv.counter) + 1;
+    double host[P * P + 1];
     sv.host = host;
     MGB_CUDA(cudaMemsetAsync(sv.counter, 0, sizeof(double), s));
-    MGB_CUDA(cudaMemsetAsync(tn, 0, sizeof(double) * (size_t)n_comp, s));
+    MGB_CUDA(cudaMemsetAsync(tn, 0, 2 * sizeof(double) * (size_t)n_comp, s));
     trivial_norm_kernel<<<sv.blocks, kSpecThreads, 0, s>>>(sd, comp, n, tn);
     MGB_LAUNCH_CHECK();
     sv.tnorm = tn;
+    double* u = static_cast<double*>(w.u.ensure((sizeof(double) + 2 * sizeof(float)) * (size_t)n));
+    float* du = reinterpret_cast<float*>(u + n);   // n ratios, n zeros (sums of t X)
+    MGB_CUDA(cudaMemsetAsync(du + n, 0, sizeof(float) * (size_t)n, s));
+    half_trivial_kernel<<<row_blocks(n), kSpecThreads, 0, s>>>(sd, n, u);
+    MGB_LAUNCH_CHECK();
+    adjoint_kernel<<<row_blocks(n * 32), kSpecThreads, 0, s>>>(indptr, indices, data, sd, comp, n, n_comp, u, open);
+    MGB_LAUNCH_CHECK();
+    ratio_kernel<<<row_blocks(n), kSpecThreads, 0, s>>>(sd, u, n, du, open);
+    MGB_LAUNCH_CHECK();
+    sv.du = du;
     sv.run(X, n_wanted, degree, max_iter, tol, w);
 }
 

@@ -10,9 +10,10 @@ namespace mgb {
 constexpr int kSpecMaxCols = 8;   // columns of the block (n_wanted + extra) the device solver takes
 
 // device scratch of the solver: the block and its filter iterate, each as it is and scaled by D^-1/2 (n x p FP64
-// each), per-component sums (three sets) and per-block partial sums
+// each), the product of a step in two launches (graphs that need it only), the weights of the projections,
+// per-component sums (three sets) and per-block partial sums
 struct SpecWork {
-    DevBuf X, Z, Y, Ynew, proj, tnorm, part;
+    DevBuf X, Z, Y, Ynew, M, u, proj, tnorm, part;
 };
 
 // X (n x p, device FP32, in and out): the start block in, the Ritz vectors out (columns by descending Ritz value).
