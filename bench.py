@@ -393,7 +393,7 @@ def config_leg(cfg, impl, steps, warmup):
 def config4_leg(impl, steps, warmup, count=256, n_iter=500):
     """the batched form: `count` independent perplexity-30 t-SNE layouts of 500-20,000 points, 500 iterations each
     (166 of early exaggeration 12, MAGNET's default min(250, n_iter // 3) for loss="tsne"); layouts/s of the batch
-    (one CUDA graph per iteration, the layouts as branches, launch shapes from the autotuner) beside the plain device
+    (one CUDA graph per iteration, its launches over many layouts each, shapes from the autotuner) beside the plain device
     form (one optimize_tsne call per layout, in sequence), or the reference's loop of optimize_tsne calls on the
     host's cores over a size-stratified sample of the layouts (impl "reference"); per-layout KL and 15-NN on the
     sample"""
@@ -444,7 +444,7 @@ def config4_leg(impl, steps, warmup, count=256, n_iter=500):
         graphs = [(P.indptr.astype(np.int32), P.indices.astype(np.int32), P.data.astype(np.float32)) for P in Ps]
         batch = mg._native.TsneBatch(graphs, n_iter=n_iter, early_iter=early,
                                      threads_per_row=int(choice.get("threads_per_row", 0)),
-                                     branches=int(choice.get("branches", 32)))
+                                     branches=int(choice.get("branches", 2)))
         dev = torch.device("cuda", torch.cuda.current_device())
         Yd0 = [torch.from_numpy(Y).to(dev) for Y in Y0s]
         Yd = [torch.empty_like(Y) for Y in Yd0]

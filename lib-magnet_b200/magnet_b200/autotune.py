@@ -2,7 +2,8 @@
 
 What it chooses, by timing a few iterations of the batch itself on the device:
   * threads per row of the attraction (the lanes that share one point's affinity row: 1-32);
-  * branches: how many of the batch's layouts run side by side in the iteration graph.
+  * branches: whether the batch's layouts run as one set of launches or as two side by side in the iteration graph (more
+    than two are the same as two, so no other count is timed).
 What it leaves alone: the interpolation grid (box count and width). The reference chooses the box count from the
 layout's extent (box width 0.7, 20-1000 boxes, magnet/tsne.py:30-46) and that choice defines the result, so the
 batch keeps it; each layout's grid allocation is sized from its point count (64 + 2 ceil(sqrt(n)) boxes).
@@ -17,7 +18,7 @@ import time
 import numpy as np
 
 TPR = (2, 4, 8, 16)
-BRANCHES = (8, 16, 32, 64)
+BRANCHES = (1, 2)
 
 
 def cache_path():
@@ -59,7 +60,7 @@ def lookup(key):
 
 
 def tune_tsne_batch(graphs, Ys, params, iters=20, tpr=TPR, branches=BRANCHES, key=None):
-    """times `iters` iterations of the batch for each threads-per-row value (at the middle branch count), then each
+    """times `iters` iterations of the batch for each threads-per-row value (at the upper branch count), then the other
     branch count at the best of those; returns {"threads_per_row": t, "branches": b, "ms": {...}} and caches it under
     `key` (batch_key of the sizes when None)"""
     from . import _native as N

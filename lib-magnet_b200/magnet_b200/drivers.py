@@ -189,7 +189,7 @@ def optimize_tsne_batch(Ps, Ys, n_iter=500, early_iter=None, early_exaggeration=
     max(200, n_i / 12).
 
     threads_per_row / branches None: the autotuner's cached choice for this batch's shape (magnet_b200.autotune),
-    tuned now when autotune is True and nothing is cached, else 8 lanes chosen from the row length and 32 branches.
+    tuned now when autotune is True and nothing is cached, else lanes chosen from the row length and two sets.
     max_boxes: per-layout grid allocation (None: 64 + 2 ceil(sqrt(n_i)))."""
     from . import autotune as A
     if early_iter is None:
@@ -207,7 +207,7 @@ def optimize_tsne_batch(Ps, Ys, n_iter=500, early_iter=None, early_exaggeration=
         choice = A.lookup(key)
         if choice is None and autotune:
             choice = A.tune_tsne_batch(graphs, Ys, params, key=key)
-        choice = choice or {"threads_per_row": 0, "branches": 32}
+        choice = choice or {"threads_per_row": 0, "branches": 2}
         threads_per_row = choice["threads_per_row"] if threads_per_row is None else threads_per_row
         branches = choice["branches"] if branches is None else branches
     batch = N.TsneBatch(graphs, n_iter=int(n_iter), threads_per_row=int(threads_per_row), branches=int(branches),
