@@ -1091,6 +1091,7 @@ void TsneDev::run_profiled(int n_iter, cudaStream_t st, double* stage_ms, int* g
     // the reported stages: 0 bbox + grid choice (the first grid; the later ones are the last stage's), 1 twiddles (the
     // spread's), 2 kernel spectra, 3 spread, 4 forward rows, 5 columns, 6 inverse rows, 7 gather + step, 8 all
     static const int slot[6] = {3, 2, 4, 5, 6, 7};
+    GridDesc gh{};   // the last iteration's grid (its step chooses the one after)
     cudaEvent_t ev[9];
     for (auto& e : ev) MGB_CUDA(cudaEventCreate(&e));
     auto between = [&](int x, int y) {
@@ -1116,13 +1117,15 @@ void TsneDev::run_profiled(int n_iter, cudaStream_t st, double* stage_ms, int* g
                 stage_ms[0] += between(7, 8);
                 stage_ms[8] += between(7, 8);
             }
+            if (it + 1 == n_iter) {
+                MGB_CUDA(cudaMemcpyAsync(&gh, gdesc.p, sizeof(GridDesc), cudaMemcpyDeviceToHost, st));
+                MGB_CUDA(cudaStreamSynchronize(st));
+            }
             loop_iterate(a, z, &lanes, 1, st, nullptr, nullptr, nullptr, ev);
             MGB_CUDA(cudaEventSynchronize(ev[6]));
             for (int k = 0; k < 6; ++k) stage_ms[slot[k]] += between(k, k + 1);
             stage_ms[8] += between(0, 6);
         }
-        GridDesc gh;
-        MGB_CUDA(cudaMemcpy(&gh, gdesc.p, sizeof(GridDesc), cudaMemcpyDeviceToHost));
         if (grid) { grid[0] = gh.n_boxes; grid[1] = gh.N; grid[2] = gh.M; grid[3] = gh.Mh; }
     } catch (...) {
         for (auto& e : ev) cudaEventDestroy(e);
