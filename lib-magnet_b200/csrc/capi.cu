@@ -33,6 +33,16 @@ Stage& stage() {
     if (!g_stage) g_stage.reset(new Stage());
     return *g_stage;
 }
+// The partial sums of the calls that reduce over a layout, of the same size from the first such call on: more than any of
+// them takes (65 doubles a block, 8 blocks per SM). A buffer that grew with a call would be an allocation inside the
+// caller's stream capture, and would be freed under a graph captured before.
+constexpr size_t kScratchBytes = (size_t)1 << 20;
+static_assert(kScratchBytes >= 1024 + sizeof(double) * (kMaxDim + 1) * 8 * kNumSMs, "the largest call's partial sums");
+DevBuf& layout_scratch() {
+    DevBuf& b = stage().scratch;
+    b.ensure(kScratchBytes);
+    return b;
+}
 
 template <class F>
 int guard(F&& f) {
@@ -319,8 +329,8 @@ static int step_impl(float* Y, float* update, float* gains, const float* A, cons
         float* Gd = in_dev(gains, t, 2, s);
         const float* Ad = in_dev(A, t, 3, s);
         const float* Fd = fused ? in_dev(F, t, 4, s) : nullptr;
-        if (fused) tsne_step_dev(Yd, Ud, Gd, Ad, Fd, n, dim, rho, inv_sumQ, lr, momentum, stage().scratch, s);
-        else tsne_update_dev(Yd, Ud, Gd, Ad, n, dim, lr, momentum, stage().scratch, s);
+        if (fused) tsne_step_dev(Yd, Ud, Gd, Ad, Fd, n, dim, rho, inv_sumQ, lr, momentum, layout_scratch(), s);
+        else tsne_update_dev(Yd, Ud, Gd, Ad, n, dim, lr, momentum, layout_scratch(), s);
         back(Y, Yd, t, s); back(update, Ud, t, s); back(gains, Gd, t, s);
         if (any_host({Y, update, gains, A, F})) MGB_CUDA(cudaStreamSynchronize(s));
     });
@@ -342,7 +352,7 @@ extern "C" int mg_bbox_2d(const float* Y, int64_t n, float* out4) {
         cudaStream_t s = current_stream();
         const float* Yd = in_dev(Y, 2 * n, 0, s);
         float* od = out_dev(out4, 4, 1);
-        bbox_dev(Yd, n, od, stage().scratch, s);
+        bbox_dev(Yd, n, od, layout_scratch(), s);
         back(out4, od, 4, s);
         if (any_host({Y, out4})) MGB_CUDA(cudaStreamSynchronize(s));
     });
@@ -395,7 +405,7 @@ void tsne_prepare(TsneDev& d, const int32_t* indptr, const int32_t* indices, con
     // P / P.sum() (magnet/tsne.py:149-150)
     if (nnz > 0) {
         const int blocks = 2 * kNumSMs;
-        char* base = static_cast<char*>(stage().scratch.ensure(64 + sizeof(double) * (blocks + 1)));
+        char* base = static_cast<char*>(layout_scratch().ensure(64 + sizeof(double) * (blocks + 1)));
         unsigned* counter = reinterpret_cast<unsigned*>(base);
         double* sum = reinterpret_cast<double*>(base + 8);
         double* part = reinterpret_cast<double*>(base + 16);
@@ -455,7 +465,7 @@ extern "C" int mg_center_scale(float* Y, int64_t n, int dim, double target_std) 
         require(Y && n >= 1 && dim >= 1 && dim <= kMaxDim, "Y must be (n, dim)");
         cudaStream_t s = current_stream();
         float* Yd = in_dev(Y, n * dim, 0, s);
-        center_scale_dev(Yd, n, dim, target_std, stage().scratch, s);
+        center_scale_dev(Yd, n, dim, target_std, layout_scratch(), s);
         back(Y, Yd, n * dim, s);
         if (!is_device_ptr(Y)) MGB_CUDA(cudaStreamSynchronize(s));
     });
