@@ -796,12 +796,13 @@ int resident_blocks(K kernel) {
 
 int env_int(const char* name, int dflt);
 
-// Lanes per walker: eight up to one and a half waves of them (nine blocks per SM; about 85,000 points), above, where the
-// thread form's warps hide each other's latency, one. us per epoch with one and with eight: 3,000 points 59 and 31, 10,000
-// 64 and 31, 47,000 72 and 42, 90,000 83 and 77, 200,000 102 and 146.
+// Lanes per walker: eight up to two waves of them (twelve blocks per SM; about 114,000 points), above, where the thread
+// form's warps hide each other's latency, one. us per epoch with one and with eight: 3,000 points 59 and 30, 10,000 64 and
+// 32, 47,000 72 and 42, 85,000 81 and 74, 100,000 84 and 80, 110,000 86 and 82, 120,000 87 and 86, 140,000 90 and 110,
+// 200,000 100 and 144.
 int walker_lanes(const SgdDev& c, int64_t threads) {
     if (c.optimizer == 1) return 1;
-    return threads * kLanes <= (int64_t)9 * kSplitBlock * kNumSMs ? kLanes : 1;
+    return threads * kLanes <= (int64_t)12 * kSplitBlock * kNumSMs ? kLanes : 1;
 }
 
 template <int D, bool FAST>

@@ -1,5 +1,5 @@
-"""The sample pass of large layouts (one thread per walker), at sizes a test can hold: n / 1 walkers at 25,011 points (more walkers
-than its eight-lane form takes: positions read as they are needed) and n / 8 at 181,003 (few enough walkers for their
+"""The sample pass of large layouts (one thread per walker), at sizes a test can hold: n / 1 walkers at 30,011 points (more walkers
+than its eight-lane form takes: positions read as they are needed) and n / 8 at 232,003 (few enough walkers for their
 points that positions are read a sample ahead). The displacement check of the sample lists: at a step size so small that
 positions stay where they are to first order, the displacement is the sum of every sample's steps at the starting
 positions. Steps of 3e-5 |g| on coordinates up to 2: a step's rounding is below 1 % of it (6e-8 / 1e-5) and averages out,
@@ -16,16 +16,16 @@ ALPHA, A, RATE, GAMMA = 3e-5, 1.7, 5.0, 1.0
 
 #        n / walkers, n, edges a row, dim, b, rep_b, mid-range pairs, b of its own per node
 CASES = {
-    "plain": (1, 25011, 7, 2, 0.8, 1.0, False, False),
-    "plain_b1": (1, 25011, 7, 2, 1.0, 1.0, False, False),
-    "plain_rep": (1, 25011, 7, 2, 0.8, 0.9, True, False),
-    "plain_3d": (1, 25011, 7, 3, 1.0, 0.9, False, False),
-    "plain_node_b": (1, 25011, 7, 2, 0.8, 1.0, False, True),
-    "ahead": (8, 181003, 4, 2, 0.8, 1.0, False, False),
-    "ahead_b1": (8, 181003, 4, 2, 1.0, 1.0, True, False),
-    "ahead_rep": (8, 181003, 4, 2, 1.0, 0.9, False, False),
-    "ahead_3d": (8, 181003, 4, 3, 0.8, 0.9, False, False),
-    "ahead_node_b": (8, 181003, 4, 3, 0.8, 1.0, True, True),
+    "plain": (1, 30011, 7, 2, 0.8, 1.0, False, False),
+    "plain_b1": (1, 30011, 7, 2, 1.0, 1.0, False, False),
+    "plain_rep": (1, 30011, 7, 2, 0.8, 0.9, True, False),
+    "plain_3d": (1, 30011, 7, 3, 1.0, 0.9, False, False),
+    "plain_node_b": (1, 30011, 7, 2, 0.8, 1.0, False, True),
+    "ahead": (8, 232003, 4, 2, 0.8, 1.0, False, False),
+    "ahead_b1": (8, 232003, 4, 2, 1.0, 1.0, True, False),
+    "ahead_rep": (8, 232003, 4, 2, 1.0, 0.9, False, False),
+    "ahead_3d": (8, 232003, 4, 3, 0.8, 0.9, False, False),
+    "ahead_node_b": (8, 232003, 4, 3, 0.8, 1.0, True, True),
 }
 
 
