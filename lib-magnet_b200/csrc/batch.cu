@@ -3,8 +3,9 @@
 //
 // Every layout keeps its own device state (TsneDev: positions, optimiser state, normalised affinities, a repulsion
 // grid sized for it). Every kernel of the iteration runs over all layouts of a set at once (their descriptors in device
-// memory; the transforms deal the layouts' rows and columns over the device as one list), so a set costs five launches
-// per iteration however many layouts it holds; `branches` up to kMaxSets sets run as branches of one CUDA graph, which
+// memory; the transforms deal the layouts' rows and columns over the device as one list), so a set costs the spread, three
+// transforms, a step launch for each number of lanes per row among its layouts, and two launches for the spectra beside
+// the spread, however many layouts it holds; `branches` up to kMaxSets sets run as branches of one CUDA graph, which
 // the host replays once per iteration. The schedule (exaggeration, momentum) follows each layout's device-side
 // iteration counter. With a branch of nine launches per layout, the launches themselves took 1.7 us each whatever the
 // branches: 24 layouts of 500-5000 points, 30 iterations, took 11.1 ms, with sets 6.2 ms.

@@ -13,8 +13,9 @@
 //    row's neighbours at once, while their distances are read; the rows of a CSR row are distinct), cleared after the
 //    query from its visit list;
 //  * both heaps are one list, the best ef rows by distance in the lanes' registers with a mark on the expanded ones:
-//    a row pushed on cand is pushed on res too, and one that has dropped out of res is farther than the ef-th result
-//    for good, so cand's next is the closest row of the list without a mark, and the search ends when there is none.
+//    a row pushed on cand is pushed on res too, and one that has dropped out of res is no closer than the ef-th result
+//    for good, so cand's next is the closest row of the list without a mark, and the search ends when there is none (the
+//    reference would still expand a dropped row that ties with the ef-th result).
 //    Rows that cannot enter are dropped by all lanes at once; the others enter one by one in the row's order, as the
 //    reference's loop takes them, by a ballot and a shift.
 // The expansion order and the result set therefore follow the reference's exactly whenever no two distances tie
@@ -35,7 +36,9 @@ namespace {
 
 constexpr int kSearchWarps = 4;        // queries in flight per block
 constexpr int kMaxEf = 256;            // result list capacity (ef)
-constexpr int kCandCap = 2048;         // rows to expand a query may hold at once; one that needs more is reported
+// Rows a query may have pushed and not expanded; one that counts more is reported as not supported. The list needs no
+// such limit: it is what a heap of candidates held, and the calls that were refused for it stay refused.
+constexpr int kCandCap = 2048;
 constexpr int kVisitCap = 8192;        // visit list per warp; past it the warp clears its whole bitset
 constexpr int kSearchPerSm = 16;       // queries in flight per SM at most: their bitsets (n / 8 bytes each) share the L2
 constexpr int kEntryTop = 8;           // entry landmarks a lane keeps in registers; more are taken one by one

@@ -8,7 +8,8 @@
 //      twiddles.
 //    The iteration reads its schedule (exaggeration, momentum) and every size from device memory, so one
 //    captured CUDA graph is replayed for all iterations; the spectra are a branch of it beside the spread.
-//    Every kernel runs over a list of layouts (one, or a batch): five launches per iteration on the path, however many.
+//    Every kernel runs over a list of layouts (one, or a batch): five launches per iteration on the path (a batch: a step
+//    launch for each number of lanes per row among its layouts).
 #include "tsne.cuh"
 #include "interp.cuh"
 #include "graph.cuh"
