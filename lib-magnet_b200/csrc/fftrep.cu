@@ -430,33 +430,40 @@ __global__ void transpose_spectra_kernel(const float* __restrict__ K, float* __r
     }
 }
 
-// the caller's grid, and the scale of the charges from the points' largest coordinates (the last block writes both)
-__global__ void __launch_bounds__(256) set_grid_kernel(GridDesc* gd, const float2* __restrict__ Y, int64_t n, float xmin,
-                                                       float ymin, float width, int n_boxes, int ni, int M, bool in_place) {
+// The caller's grid, and the scale of the charges from the points' largest coordinates. Up to kGridPoints points one block
+// takes them; more blocks leave their maxima to the last one. (A plain call waits for this launch: it is latency.)
+constexpr int kGridThreads = 1024;
+constexpr int kGridPoints = 16 * kGridThreads;
+__global__ void __launch_bounds__(kGridThreads) set_grid_kernel(GridDesc* gd, const float2* __restrict__ Y, int64_t n, float xmin,
+                                                                float ymin, float width, int n_boxes, int ni, int M,
+                                                                bool in_place) {
     __shared__ unsigned peak[2];
-    __shared__ int is_last;
     if (threadIdx.x < 2) peak[threadIdx.x] = 0u;
     float ax = 0.f, ay = 0.f;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const float2 p = Y[i];
-        ax = fmaxf(ax, fabsf(p.x)); ay = fmaxf(ay, fabsf(p.y));
+    const int64_t step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += 8 * step) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {   // reads under way together
+            const float2 p = i + q * step < n ? Y[i + q * step] : make_float2(0.f, 0.f);
+            ax = fmaxf(ax, fabsf(p.x)); ay = fmaxf(ay, fabsf(p.y));
+        }
     }
     __syncthreads();
     const unsigned mx = __reduce_max_sync(0xffffffffu, __float_as_uint(ax));
     const unsigned my = __reduce_max_sync(0xffffffffu, __float_as_uint(ay));
     if ((threadIdx.x & 31) == 0) { atomicMax(&peak[0], mx); atomicMax(&peak[1], my); }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x != 0) return;
+    ax = __uint_as_float(peak[0]); ay = __uint_as_float(peak[1]);
+    if (gridDim.x > 1) {
         atomicMax(&gd->peak[0], peak[0]);
         atomicMax(&gd->peak[1], peak[1]);
         __threadfence();
-        is_last = atomicAdd(&gd->counter2, 1u) == gridDim.x - 1;
+        if (atomicAdd(&gd->counter2, 1u) != gridDim.x - 1) return;
+        __threadfence();
+        ax = __uint_as_float(__ldcg(&gd->peak[0])); ay = __uint_as_float(__ldcg(&gd->peak[1]));
+        gd->peak[0] = 0u; gd->peak[1] = 0u; gd->counter2 = 0u;
     }
-    __syncthreads();
-    if (!is_last || threadIdx.x != 0) return;
-    __threadfence();
-    ax = __uint_as_float(__ldcg(&gd->peak[0])); ay = __uint_as_float(__ldcg(&gd->peak[1]));
-    gd->peak[0] = 0u; gd->peak[1] = 0u; gd->counter2 = 0u;
     if (in_place) set_field_scale(gd, ax, ay);
     else gd->up = gd->down = make_float2(1.f, 1.f);
     gd->xmin = xmin; gd->ymin = ymin; gd->width = width; gd->inv_width = 1.f / width;
@@ -492,8 +499,10 @@ void gather_t(const float2* Y, int64_t n, GridDesc* g, RepBuffers& b, float2* F,
 
 void rep_set_grid(GridDesc* g_dev, const float2* Y, int64_t n, float xmin, float ymin, float width, int n_boxes, int ni,
                   int M, bool in_place, cudaStream_t s) {
-    const int blocks = in_place ? (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 4 * kNumSMs)) : 1;
-    set_grid_kernel<<<blocks, 256, 0, s>>>(g_dev, Y, in_place ? n : 0, xmin, ymin, width, n_boxes, ni, M, in_place);
+    const int64_t points = in_place ? n : 0;
+    const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((points + kGridPoints - 1) / kGridPoints, kNumSMs));
+    const int threads = (int)std::min<int64_t>(kGridThreads, std::max<int64_t>(32, (points + 31) / 32 * 32));
+    set_grid_kernel<<<blocks, threads, 0, s>>>(g_dev, Y, points, xmin, ymin, width, n_boxes, ni, M, in_place);
     MGB_LAUNCH_CHECK();
 }
 
